@@ -188,31 +188,95 @@ __device__ void stage_p(const C *__restrict__ src, C *__restrict__ dst, int n, i
     }
 }
 
-// Generic radix (direct size-p DFT per butterfly, O(p^2)).
+// Generic radix p (a prime >= 7, in practice a large factor of a ragged grid),
+// O(p) work per output, every output its own thread's: a butterfly's p^2
+// products are spread over the block (one thread per butterfly left 2 of 256
+// threads busy on 386 = 2 x 193).  The inputs are twiddled in place first, so
+// no output repeats that product.
+//
+// FP64 is bound by the FP64 pipe (2 lanes per clock and SM), so it folds the
+// symmetric inputs, S_t = x_t + x_{p-t} and D_t = x_t - x_{p-t}, in place
+// (S_t at t, D_t at p - t) and forms the outputs j and p - j together,
+//   X_{j, p-j} = (x_0 + sum_t S_t cos(2 pi j t / p)) +/- i (sum_t D_t sin(2 pi j t / p)):
+// a quarter of the direct sum's FMAs, and fewer roundings.  FP32 keeps the
+// direct sum in its order.
 template <typename C, int SIGN>
-__device__ void stage_generic(const C *__restrict__ src, C *__restrict__ dst, int n, int nlines, int L1, int p,
-                              int rq, const FDiv drq, const FDiv dnb, const C *__restrict__ tw)
+__device__ void stage_generic(C *__restrict__ src, C *__restrict__ dst, int n, int nlines, int L1, int p, int rq,
+                              const FDiv drq, const FDiv dnb, const C *__restrict__ tw)
 {
+    typedef decltype(src[0].x) RR;
     const int nb = n / p;
-    const int total = nb * nlines;
     const int np_ = n / p;
-    for (int b = threadIdx.x; b < total; b += blockDim.x) {
-        const int line = (int)fdiv((uint32_t)b, dnb);
-        const int loc = b - line * nb;
-        const int j1 = (int)fdiv((uint32_t)loc, drq);
-        const int k = loc - j1 * rq;
-        const C *s = src + (size_t)line * n;
-        C *d = dst + (size_t)line * n;
-        const int base = j1 * rq * p + k;
-        for (int j2 = 0; j2 < p; ++j2) {
-            C acc = s[base];
-            for (int t = 1; t < p; ++t) {
-                C v = s[base + t * rq];
-                if (j1 > 0) v = cx_mul(v, tw_get<C, SIGN>(tw, j1 * t * rq));
-                int m = ((j2 * t) % p) * np_;
-                acc = cx_add(acc, cx_mul(v, tw_get<C, SIGN>(tw, m)));
+    if constexpr (sizeof(RR) == 8) {
+        const int h = p >> 1, bl = nb * nlines;  // p is odd
+        for (int b = threadIdx.x; b < bl * h; b += blockDim.x) {
+            const int t = 1 + b / bl, bb = b - (t - 1) * bl;  // consecutive threads: consecutive butterflies
+            const int line = (int)fdiv((uint32_t)bb, dnb);
+            const int loc = bb - line * nb;
+            const int j1 = (int)fdiv((uint32_t)loc, drq);
+            C *s = src + (size_t)line * n + j1 * rq * p + (loc - j1 * rq);
+            C x = s[t * rq], y = s[(p - t) * rq];
+            if (j1 > 0) {
+                x = cx_mul(x, tw_get<C, SIGN>(tw, j1 * t * rq));
+                y = cx_mul(y, tw_get<C, SIGN>(tw, j1 * (p - t) * rq));
             }
-            d[(j1 + L1 * j2) * rq + k] = acc;
+            s[t * rq] = cx_add(x, y);
+            s[(p - t) * rq] = cx_sub(x, y);
+        }
+        __syncthreads();
+        for (int b = threadIdx.x; b < bl * (h + 1); b += blockDim.x) {
+            const int j = b / bl, bb = b - j * bl;
+            const int line = (int)fdiv((uint32_t)bb, dnb);
+            const int loc = bb - line * nb;
+            const int j1 = (int)fdiv((uint32_t)loc, drq);
+            const int k = loc - j1 * rq;
+            const C *s = src + (size_t)line * n + j1 * rq * p + k;
+            C *d = dst + (size_t)line * n + k;
+            C A = s[0], B = cx_make<C>(0.0, 0.0);
+            int m = 0;
+            for (int t = 1; t <= h; ++t) {
+                m += j;
+                if (m >= p) m -= p;
+                const C w = tw[m * np_];  // (cos, -sin)
+                const C S = s[t * rq], D = s[(p - t) * rq];
+                A.x = fma(S.x, w.x, A.x);
+                A.y = fma(S.y, w.x, A.y);
+                B.x = fma(D.x, w.y, B.x);
+                B.y = fma(D.y, w.y, B.y);
+            }
+            // i SIGN (-B): the table holds -sin
+            const C r = cx_rot(B, (float)-SIGN);
+            d[(j1 + L1 * j) * rq] = cx_add(A, r);
+            if (j > 0) d[(j1 + L1 * (p - j)) * rq] = cx_sub(A, r);
+        }
+    } else {
+        const int bl = nb * nlines;
+        if (L1 > 1) {
+            for (int b = threadIdx.x; b < bl * (p - 1); b += blockDim.x) {
+                const int t = 1 + b / bl, bb = b - (t - 1) * bl;
+                const int line = (int)fdiv((uint32_t)bb, dnb);
+                const int loc = bb - line * nb;
+                const int j1 = (int)fdiv((uint32_t)loc, drq);
+                C *s = src + (size_t)line * n + j1 * rq * p + (loc - j1 * rq);
+                if (j1 > 0) s[t * rq] = cx_mul(s[t * rq], tw_get<C, SIGN>(tw, j1 * t * rq));
+            }
+            __syncthreads();
+        }
+        for (int b = threadIdx.x; b < bl * p; b += blockDim.x) {
+            const int j2 = b / bl, bb = b - j2 * bl;
+            const int line = (int)fdiv((uint32_t)bb, dnb);
+            const int loc = bb - line * nb;
+            const int j1 = (int)fdiv((uint32_t)loc, drq);
+            const int k = loc - j1 * rq;
+            const C *s = src + (size_t)line * n + j1 * rq * p + k;
+            C acc = s[0];
+            int m = 0;
+            for (int t = 1; t < p; ++t) {
+                m += j2;
+                if (m >= p) m -= p;
+                acc = cx_add(acc, cx_mul(s[t * rq], tw_get<C, SIGN>(tw, m * np_)));
+            }
+            dst[(size_t)line * n + (j1 + L1 * j2) * rq + k] = acc;
         }
     }
 }
