@@ -2,14 +2,21 @@
 // src/bldfm/utils.py:80-92, np.sum(f * g)) for a batch of (footprint, flux)
 // pairs: out[b] = sum_i f[b][i] g[b][i] in FP64.
 //
-// The field is HBM-bound (16 bytes read per point, nothing written): each
-// batch entry is split over the CTAs of one grid row, every thread keeps a
-// Kahan-compensated FP64 sum of its grid-stride points (16-byte vector loads
-// where the arrays allow), the CTA combines its threads in a fixed tree
-// order, and a second kernel adds the per-CTA partials in index order, so the
-// result is deterministic (no atomics) and carries about eps of error
-// independent of n; numpy's pairwise sum differs from it at the level of its
-// own rounding (about log2(n) eps).
+// The field is HBM-bound (16 bytes read per point, nothing written) as long as
+// the FP64 pipe keeps up: at 2 lanes per clock and SM it passes about 0.53 T
+// instructions/s, while HBM delivers 0.42 T points/s, so a point may cost no
+// more than 1.25 FP64 instructions.  A compensated sum per point took five
+// (195 us for 64 x 512^2 points, 1.37 TB/s).  Here a thread adds 16 points in
+// two chains of 8 FMAs (products unrounded) and only the sum of those 16 goes
+// through the compensated accumulator: 1.31 instructions a point.  The short
+// chains' roundings are independent and average out over the blocks; the
+// result's error stays at the rounding of its last additions.  Each batch
+// entry is split over the CTAs of one grid row, each with a contiguous range;
+// the CTA combines its threads in a fixed tree order, and a second kernel (one
+// warp per entry) adds the per-CTA partials in a fixed order, so the result is
+// deterministic (no atomics) and carries about eps of error independent of n;
+// numpy's pairwise sum differs from it at the level of its own rounding (about
+// log2(n) eps).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -31,27 +38,53 @@ struct Kahan {
     }
 };
 
-__global__ void __launch_bounds__(MEAS_THREADS) meas_partial_kernel(const double *__restrict__ f,
-                                                                    const double *__restrict__ g, int64_t n,
-                                                                    int64_t stride, double *__restrict__ part)
+const int MEAS_UNROLL = 8;  // 16-byte loads of each field in flight per thread
+const int MEAS_CTAS = 4;    // resident CTAs per SM the grid is sized for (at most 64 registers a thread)
+
+__global__ void __launch_bounds__(MEAS_THREADS, MEAS_CTAS)
+    meas_partial_kernel(const double *__restrict__ f, const double *__restrict__ g, int64_t n, int64_t stride,
+                        double *__restrict__ part)
 {
     const int b = blockIdx.y;
     const double *fb = f + (size_t)b * stride, *gb = g + (size_t)b * stride;
     Kahan k;
-    const int64_t t0 = (int64_t)blockIdx.x * MEAS_THREADS + threadIdx.x;
-    const int64_t step = (int64_t)gridDim.x * MEAS_THREADS;
-    const bool vec = ((((uintptr_t)fb) | ((uintptr_t)gb)) & 15) == 0;
+    const bool vec = ((((uintptr_t)fb) ^ ((uintptr_t)gb)) & 15) == 0;
     if (vec) {
-        const int64_t n2 = n / 2;
-        const double2 *f2 = (const double2 *)fb, *g2 = (const double2 *)gb;
-        for (int64_t i = t0; i < n2; i += step) {
-            const double2 a = __ldg(f2 + i), c = __ldg(g2 + i);
-            k.add(__dmul_rn(a.x, c.x));
-            k.add(__dmul_rn(a.y, c.y));
+        // both at the same 8-byte phase: one leading point at most, then pairs
+        const int lead = (((uintptr_t)fb) & 15) != 0 && n > 0 ? 1 : 0;
+        const int64_t n2 = (n - lead) / 2;
+        const double2 *f2 = (const double2 *)(fb + lead), *g2 = (const double2 *)(gb + lead);
+        // this CTA's pairs
+        const int64_t per = (n2 + gridDim.x - 1) / gridDim.x;
+        const int64_t lo = (int64_t)blockIdx.x * per, hi = min(n2, lo + per);
+        int64_t i = lo + threadIdx.x;
+        for (; i + (MEAS_UNROLL - 1) * MEAS_THREADS < hi; i += MEAS_UNROLL * MEAS_THREADS) {
+            double2 a[MEAS_UNROLL], c[MEAS_UNROLL];
+#pragma unroll
+            for (int u = 0; u < MEAS_UNROLL; ++u) {
+                a[u] = __ldcs(f2 + i + u * MEAS_THREADS);
+                c[u] = __ldcs(g2 + i + u * MEAS_THREADS);
+            }
+            double s0 = a[0].x * c[0].x, s1 = a[0].y * c[0].y;
+#pragma unroll
+            for (int u = 1; u < MEAS_UNROLL; ++u) {
+                s0 = fma(a[u].x, c[u].x, s0);
+                s1 = fma(a[u].y, c[u].y, s1);
+            }
+            k.add(__dadd_rn(s0, s1));
         }
-        if ((n & 1) && t0 == 0) k.add(__dmul_rn(fb[n - 1], gb[n - 1]));
+        for (; i < hi; i += MEAS_THREADS) {
+            const double2 a = __ldcs(f2 + i), c = __ldcs(g2 + i);
+            k.add(fma(a.x, c.x, __dmul_rn(a.y, c.y)));
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (lead) k.add(__dmul_rn(fb[0], gb[0]));
+            if ((n - lead) & 1) k.add(__dmul_rn(fb[n - 1], gb[n - 1]));
+        }
     } else {
-        for (int64_t i = t0; i < n; i += step) k.add(__dmul_rn(__ldg(fb + i), __ldg(gb + i)));
+        const int64_t step = (int64_t)gridDim.x * MEAS_THREADS;
+        for (int64_t i = (int64_t)blockIdx.x * MEAS_THREADS + threadIdx.x; i < n; i += step)
+            k.add(__dmul_rn(__ldg(fb + i), __ldg(gb + i)));
     }
     __shared__ double ss[MEAS_THREADS];
     ss[threadIdx.x] = __dadd_rn(k.s, -k.c);
@@ -63,13 +96,20 @@ __global__ void __launch_bounds__(MEAS_THREADS) meas_partial_kernel(const double
     if (threadIdx.x == 0) part[(size_t)b * gridDim.x + blockIdx.x] = ss[0];
 }
 
-__global__ void meas_final_kernel(const double *__restrict__ part, int nparts, int nbatch, double *__restrict__ out)
+// One warp per batch entry: lane l adds the partials l, l + 32, ... (one
+// thread's chain over all 600 partials of a single field took longer than the
+// field's own pass), then the lanes in a fixed tree order.
+__global__ void __launch_bounds__(128) meas_final_kernel(const double *__restrict__ part, int nparts, int nbatch,
+                                                         double *__restrict__ out)
 {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nbatch) return;
     Kahan k;
-    for (int i = 0; i < nparts; ++i) k.add(part[(size_t)b * nparts + i]);
-    out[b] = __dadd_rn(k.s, -k.c);
+    for (int i = lane; i < nparts; i += 32) k.add(part[(size_t)b * nparts + i]);
+    double s = __dadd_rn(k.s, -k.c);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s = __dadd_rn(s, __shfl_down_sync(0xffffffffu, s, off));
+    if (lane == 0) out[b] = s;
 }
 
 // One CTA waits on an mbarrier that nothing arrives at, with an iteration
@@ -136,8 +176,9 @@ int64_t bldfm_point_measurement_workspace(int64_t n, int32_t nbatch)
     if (n < 0 || nbatch < 1) return -1;
     int dev = 0, nsm = 152;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    int64_t per = (n + MEAS_THREADS * 8 - 1) / (MEAS_THREADS * 8);
-    const int64_t want = (int64_t)nsm * 4 / nbatch + 1;
+    // CTAs per entry: enough points for each, and one wave over the device
+    int64_t per = (n + MEAS_THREADS * 4 - 1) / (MEAS_THREADS * 4);
+    const int64_t want = (int64_t)nsm * MEAS_CTAS / nbatch;
     if (per > want) per = want;
     if (per < 1) per = 1;
     if (per > 65535) per = 65535;
@@ -155,7 +196,7 @@ int bldfm_point_measurement(const double *f_dev, const double *g_dev, int64_t n,
     cudaStream_t st = (cudaStream_t)stream;
     double *part = (double *)workspace_dev;
     meas_partial_kernel<<<dim3(per, nbatch), MEAS_THREADS, 0, st>>>(f_dev, g_dev, n, stride, part);
-    meas_final_kernel<<<(nbatch + 127) / 128, 128, 0, st>>>(part, per, nbatch, out_dev);
+    meas_final_kernel<<<(nbatch + 3) / 4, 128, 0, st>>>(part, per, nbatch, out_dev);
     return cudaGetLastError() == cudaSuccess ? BLDFM_OK : BLDFM_ERR_CUDA;
 }
 

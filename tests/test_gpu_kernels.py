@@ -1,0 +1,65 @@
+"""Kernels at the sizes where their tiling can go wrong: prime factors of the
+transform lengths, remainders and alignments of the point measurement."""
+
+import math
+
+import numpy as np
+import pytest
+
+from oracle import bldfm_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def relerr(a, b):
+    return float(np.linalg.norm(np.asarray(a, np.float64) - b) / np.linalg.norm(b))
+
+
+def ragged_kw(nx, ny, halo_cells, footprint, n=6):
+    """A solve whose extended grid is (nx, ny) + 2 halo_cells with unit cells."""
+    z, p = O.vertical_profiles(n, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    rng = np.random.default_rng(nx * 1000 + ny)
+    src = np.zeros((ny, nx)) if footprint else rng.uniform(0.0, 1.0, (ny, nx))
+    return dict(srf_flx=src, z=z, profiles=p, domain=(float(nx), float(ny)), levels=n, modes=(nx & ~1, ny & ~1),
+                meas_pt=(3.0, 2.0), footprint=footprint, halo=halo_cells + 0.5, precision="double")
+
+
+@pytest.mark.parametrize("nx,ny,halo,footprint", [
+    (14, 22, 0, True), (14, 22, 0, False),     # 2 x 7, 2 x 11: the smallest generic factors
+    (10, 26, 13, False),                       # 36 and 52 = 4 x 13
+    (59, 129, 129, True),                      # output lines 316 = 4 x 79 and 386 = 2 x 193
+    (30, 34, 114, False),                      # 258 = 2 x 3 x 43 and 262 = 2 x 131
+    (98, 50, 0, False),                        # 2 x 7 x 7: two generic stages
+])
+def test_generic_radix_lengths(nx, ny, halo, footprint):
+    """FP64 solves on lines with large prime factors against the oracle (numpy's
+    FFT): the bar of the FP64 path, 1e-10."""
+    from bldfm_gb300 import steady_state_transport_solver
+
+    kw = ragged_kw(nx, ny, halo, footprint)
+    _, c, f = steady_state_transport_solver(**kw)
+    _, oc, of = O.steady_state_transport_solver(**kw)
+    assert relerr(c, oc) <= 1e-10 and relerr(f, of) <= 1e-10
+    _, c32, f32 = steady_state_transport_solver(**kw, mode="fp32")
+    assert relerr(c32, oc) <= 1e-4 and relerr(f32, of) <= 1e-4
+
+
+@pytest.mark.parametrize("count,n", [(1, 1), (1, 2), (3, 1023), (2, 1024), (5, 4095), (3, 4097), (2, 70001),
+                                     (700, 33), (1, 1300003)])
+@pytest.mark.parametrize("phase", [0, 1])
+def test_point_measurement_remainders(count, n, phase):
+    """Every remainder and both 8-byte phases against math.fsum of the exact
+    products' roundings: a few eps of the sum of magnitudes."""
+    import torch
+
+    from bldfm_gb300.utils import point_measurement_batch
+
+    rng = np.random.default_rng(n)
+    F = rng.standard_normal(count * n + 1)
+    G = rng.standard_normal(count * n + 1)
+    f = torch.from_numpy(F).cuda()[phase:phase + count * n].view(count, n)
+    g = torch.from_numpy(G).cuda()[phase:phase + count * n].view(count, n)
+    out = point_measurement_batch(f, g).cpu().numpy()
+    for b in range(0, count, max(1, count // 7)):
+        a = F[phase + b * n:phase + (b + 1) * n] * G[phase + b * n:phase + (b + 1) * n]
+        assert abs(out[b] - math.fsum(a)) <= 4 * 2.0**-52 * math.fsum(np.abs(a))
