@@ -17,6 +17,7 @@
 #include "profiles.h"
 #include "surrogate_phys.cuh"
 #include "tcgemm.cuh"
+#include "train.h"
 
 namespace {
 
@@ -106,41 +107,12 @@ extern "C" int bldfm_tc_gemm_check(const uint16_t *A, const uint16_t *B, float *
 namespace {
 
 // A CTA's 128 x 256 bf16 tile in core-matrix order (tc_core_offset) is copied
-// to the row blocks of its tile (contiguous 64 KB), and scattered into the
-// transposed layouts used as operands of the weight-gradient GEMM:
-//   mode 0 (B operand, H^T): blocks [chunk = sample / 256] of 256 x 256,
-//          element (feature, sample % 256)
-//   mode 1 (A operand, dZ^T): blocks [feature / 128][chunk] of 128 x 256,
-//          element (feature % 128, sample % 256)
-__device__ void emit_tile(int tile, const uint16_t *st, uint16_t *rows_dst, uint16_t *T_dst, int mode, int nchunks)
+// to the row block of its tile (contiguous 64 KB)
+__device__ void emit_tile(int tile, const uint16_t *st, uint16_t *rows_dst)
 {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    if (rows_dst) {
-        const uint4 *s = (const uint4 *)st;
-        uint4 *d = (uint4 *)(rows_dst + (size_t)tile * 128 * MLP_H);
-        for (int i = tid; i < 128 * MLP_H / 8; i += nt) d[i] = s[i];
-    }
-    if (!T_dst) return;
-    const int chunk = tile >> 1, half = tile & 1;
-    // one 16-byte store per (feature, group of 8 samples): 256 x 16 per tile
-    for (int i = tid; i < MLP_H * 16; i += nt) {
-        const int f = i & (MLP_H - 1), g = i >> 8;  // consecutive threads: consecutive features
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int s0 = g * 8 + 2 * q;
-            const uint32_t lo = st[tc_core_offset(s0, f, MLP_H) / 2];
-            const uint32_t hi = st[tc_core_offset(s0 + 1, f, MLP_H) / 2];
-            w[q] = lo | (hi << 16);
-        }
-        const int s256 = half * 128 + g * 8;
-        size_t off;
-        if (mode == 0)
-            off = (size_t)chunk * MLP_H * 256 + tc_core_offset(f, s256, 256) / 2;
-        else
-            off = ((size_t)(f >> 7) * nchunks + chunk) * 128 * 256 + tc_core_offset(f & 127, s256, 256) / 2;
-        *(uint4 *)(T_dst + off) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    const uint4 *s = (const uint4 *)st;
+    uint4 *d = (uint4 *)(rows_dst + (size_t)tile * 128 * MLP_H);
+    for (int i = threadIdx.x; i < 128 * MLP_H / 8; i += blockDim.x) d[i] = s[i];
 }
 
 // 8 consecutive values of one row into the smem tile (one 16-byte store)
@@ -152,43 +124,23 @@ __device__ __forceinline__ void put8(uint16_t *st, int r, int c, const float *v)
     *(uint4 *)(st + tc_core_offset(r, c, MLP_H) / 2) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// forward hidden layer: Z = acc + b, H = gelu(Z); written as the bf16 rows
-// and transposed blocks of the next GEMM (rows_dst, T_dst), gelu'(Z) as bf16
-// (G_dst), H in FP32 row-major (h32_dst), or straight into the output layer:
+// forward hidden layer: H = gelu(acc + b); written as the bf16 rows of the next
+// GEMM (rows_dst) or straight into the output layer:
 // Y[r] = b4 + sum_f H[r][f] W4[f] in FP32 (Y != null).  Null pointers skip.
 struct EpiFwd {
     const float *bias;
-    uint16_t *rows_dst, *T_dst, *G_dst;
-    float *h32_dst;
+    uint16_t *rows_dst;
     const float *W4, *b4;
     float *Y;
-    int nchunks;
     __device__ void row(int r, int c0, const float *v, uint16_t *st) const
     {
-        float h[32], gd[32];
+        float h[32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const float z = v[i] + bias[c0 + i];
-            h[i] = gelu_f(z);
-            gd[i] = G_dst ? gelu_d(z) : 0.f;
-        }
-        if (rows_dst || T_dst) {
+        for (int i = 0; i < 32; ++i) h[i] = gelu_f(v[i] + bias[c0 + i]);
+        if (rows_dst) {
             const int rl = r & 127;
 #pragma unroll
             for (int q = 0; q < 4; ++q) put8(st, rl, c0 + 8 * q, h + 8 * q);
-        }
-        if (G_dst) {
-            uint32_t w[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) w[i] = (uint32_t)f2bf(gd[2 * i]) | ((uint32_t)f2bf(gd[2 * i + 1]) << 16);
-            uint4 *g = (uint4 *)(G_dst + (size_t)r * MLP_H + c0);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) g[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-        }
-        if (h32_dst) {
-            float4 *o = (float4 *)(h32_dst + (size_t)r * MLP_H + c0);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) o[q] = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
         }
         if (Y) {
             // this thread owns row r for every column slice, in order
@@ -207,72 +159,13 @@ struct EpiFwd {
     }
     __device__ void finish(int tile, uint16_t *st) const
     {
-        if (rows_dst || T_dst) emit_tile(tile, st, rows_dst, T_dst, 0, nchunks);
+        if (rows_dst) emit_tile(tile, st, rows_dst);
     }
-};
-
-// backward data: dZ = bf16(acc * G); db += sum over rows of dZ
-struct EpiBwd {
-    const uint16_t *G;
-    uint16_t *rows_dst, *T_dst;
-    float *rowmajor_f32;  // dZ1 for the input layer's gradient
-    float *dbias;
-    int nchunks;
-    __device__ void row(int r, int c0, const float *v, uint16_t *st) const
-    {
-        float dz[32];
-        const uint4 *g4 = (const uint4 *)(G + (size_t)r * MLP_H + c0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 u = g4[q];
-            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                dz[8 * q + 2 * k] = bf2f(f2bf(v[8 * q + 2 * k] * bf2f((uint16_t)(w[k] & 0xFFFF))));
-                dz[8 * q + 2 * k + 1] = bf2f(f2bf(v[8 * q + 2 * k + 1] * bf2f((uint16_t)(w[k] >> 16))));
-            }
-        }
-        if (rows_dst || T_dst) {
-            const int rl = r & 127;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) put8(st, rl, c0 + 8 * q, dz + 8 * q);
-        }
-        if (rowmajor_f32) {
-            float4 *o = (float4 *)(rowmajor_f32 + (size_t)r * MLP_H + c0);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) o[q] = make_float4(dz[4 * q], dz[4 * q + 1], dz[4 * q + 2], dz[4 * q + 3]);
-        }
-        // bias gradient: sum the warp's 32 rows per column, one atomic per column
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            float s = dz[i];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-            if ((threadIdx.x & 31) == 0) atomicAdd(dbias + c0 + i, s);
-        }
-    }
-    __device__ void finish(int tile, uint16_t *st) const
-    {
-        if (rows_dst || T_dst) emit_tile(tile, st, rows_dst, T_dst, 1, nchunks);
-    }
-};
-
-// weight gradient partial sums: grad[out][in] += acc
-struct EpiGrad {
-    float *grad;
-    __device__ void row(int r, int c0, const float *v, uint16_t *) const
-    {
-        float *o = grad + (size_t)r * MLP_H + c0;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) atomicAdd(o + i, v[i]);
-    }
-    __device__ void finish(int, uint16_t *) const {}
 };
 
 // input layer forward: one CTA per 128-sample tile, thread = feature
 __global__ void __launch_bounds__(256) mlp_in_fwd_kernel(const float *__restrict__ X, const float *__restrict__ P,
-                                                         uint16_t *rows_dst, uint16_t *T_dst, uint16_t *G_dst,
-                                                         int nchunks)
+                                                         uint16_t *rows_dst)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t *st = (uint16_t *)smem_raw;
@@ -288,180 +181,19 @@ __global__ void __launch_bounds__(256) mlp_in_fwd_kernel(const float *__restrict
 #pragma unroll
         for (int i = 0; i < MLP_IN; ++i) z = fmaf(x[i], w[i], z);
         st[tc_core_offset(s, f, MLP_H) / 2] = f2bf(gelu_f(z));
-        if (G_dst) G_dst[(size_t)r * MLP_H + f] = f2bf(gelu_d(z));
     }
     __syncthreads();
-    emit_tile(tile, st, rows_dst, T_dst, 0, nchunks);
-}
-
-// Output layer forward, loss and the start of the backward pass: one CTA per
-// 128-sample tile.  Phase 1, thread = sample: y = H4 W4 + b4, the weighted
-// error and dY (kept in shared memory).  Phase 2, thread = two features:
-// dW4 = H4^T dY and dZ4 = bf16(dY W4^T * gelu'), db3 = sum dZ4, reduced over
-// the tile's rows in registers (one global atomic per parameter and CTA).
-__global__ void __launch_bounds__(128) mlp_out_kernel(const float *__restrict__ H4, const uint16_t *__restrict__ G4,
-                                                      const float *__restrict__ P, const float *__restrict__ T,
-                                                      const float *__restrict__ wts, float inv_n, float *Y,
-                                                      float *grad, float *loss, uint16_t *rows_dst, uint16_t *T_dst,
-                                                      int nchunks, int n)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint16_t *st = (uint16_t *)smem_raw;                // dZ4 tile (64 KB)
-    float *sW = (float *)(smem_raw + 128 * MLP_H * 2);  // W4 [256][4]
-    float4 *sDY = (float4 *)(sW + MLP_H * MLP_OUT);     // dY [128]
-    __shared__ float sdb4[MLP_OUT], sloss;
-    const int t = threadIdx.x, tile = blockIdx.x;
-    for (int i = t; i < MLP_H * MLP_OUT; i += blockDim.x) sW[i] = P[MLP_OFF_W4 + i];
-    if (t < MLP_OUT) sdb4[t] = 0.f;
-    if (t == 0) sloss = 0.f;
-    __syncthreads();
-    const int r = tile * 128 + t;
-    const bool live = r < n;
-    const float4 *h4 = (const float4 *)(H4 + (size_t)(live ? r : 0) * MLP_H);
-    float y[MLP_OUT];
-#pragma unroll
-    for (int o = 0; o < MLP_OUT; ++o) y[o] = P[MLP_OFF_B4 + o];
-    for (int q = 0; q < MLP_H / 4; ++q) {
-        const float4 u = h4[q];
-        const float hq[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int f = q * 4 + k;
-#pragma unroll
-            for (int o = 0; o < MLP_OUT; ++o) y[o] = fmaf(hq[k], sW[f * MLP_OUT + o], y[o]);
-        }
-    }
-    if (Y && live)
-        for (int o = 0; o < MLP_OUT; ++o) Y[(size_t)r * MLP_OUT + o] = y[o];
-    if (!T) return;
-    float dy[MLP_OUT];
-    float l = 0.f;
-#pragma unroll
-    for (int o = 0; o < MLP_OUT; ++o) {
-        const float wb = live ? wts[(size_t)r * MLP_OUT + o] : 0.f;
-        const float e = live ? (y[o] - T[(size_t)r * MLP_OUT + o]) : 0.f;
-        l = fmaf(wb * e, e, l);
-        dy[o] = 2.f * wb * e * inv_n;
-    }
-    sDY[t] = make_float4(dy[0], dy[1], dy[2], dy[3]);
-    // tile sums of the loss and db4: warp reductions, one shared atomic per warp
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        l += __shfl_xor_sync(0xffffffffu, l, off);
-#pragma unroll
-        for (int o = 0; o < MLP_OUT; ++o) dy[o] += __shfl_xor_sync(0xffffffffu, dy[o], off);
-    }
-    if ((t & 31) == 0) {
-        atomicAdd(&sloss, l * inv_n);
-#pragma unroll
-        for (int o = 0; o < MLP_OUT; ++o) atomicAdd(&sdb4[o], dy[o]);
-    }
-    __syncthreads();
-    // phase 2: features f0 = 2 t, f0 + 1
-    const int f0 = 2 * t;
-    float gW[2][MLP_OUT] = {};
-    float db[2] = {0.f, 0.f};
-    float w4[2][MLP_OUT];
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int o = 0; o < MLP_OUT; ++o) w4[k][o] = sW[(f0 + k) * MLP_OUT + o];
-    const int rows = min(128, n - tile * 128);
-    for (int rr = 0; rr < rows; ++rr) {
-        const size_t gr = (size_t)(tile * 128 + rr) * MLP_H + f0;
-        const float2 h = *(const float2 *)(H4 + gr);
-        const uint32_t gw = *(const uint32_t *)(G4 + gr);
-        const float4 d = sDY[rr];
-        const float hk[2] = {h.x, h.y};
-        const float gk[2] = {bf2f((uint16_t)(gw & 0xFFFF)), bf2f((uint16_t)(gw >> 16))};
-        uint16_t zb[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            gW[k][0] = fmaf(hk[k], d.x, gW[k][0]);
-            gW[k][1] = fmaf(hk[k], d.y, gW[k][1]);
-            gW[k][2] = fmaf(hk[k], d.z, gW[k][2]);
-            gW[k][3] = fmaf(hk[k], d.w, gW[k][3]);
-            const float dh = fmaf(d.x, w4[k][0], fmaf(d.y, w4[k][1], fmaf(d.z, w4[k][2], d.w * w4[k][3])));
-            zb[k] = f2bf(dh * gk[k]);
-            db[k] += bf2f(zb[k]);
-        }
-        // f0 is even, so the pair is one aligned 32-bit word of the core-matrix row
-        *(uint32_t *)(st + tc_core_offset(rr, f0, MLP_H) / 2) = (uint32_t)zb[0] | ((uint32_t)zb[1] << 16);
-    }
-    for (int rr = rows; rr < 128; ++rr) *(uint32_t *)(st + tc_core_offset(rr, f0, MLP_H) / 2) = 0u;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-#pragma unroll
-        for (int o = 0; o < MLP_OUT; ++o) atomicAdd(grad + MLP_OFF_W4 + (f0 + k) * MLP_OUT + o, gW[k][o]);
-        atomicAdd(grad + MLP_OFF_B(3) + f0 + k, db[k]);
-    }
-    if (t < MLP_OUT) atomicAdd(grad + MLP_OFF_B4 + t, sdb4[t]);
-    if (t == 0) atomicAdd(loss, sloss);
-    __syncthreads();
-    emit_tile(tile, st, rows_dst, T_dst, 1, nchunks);
-}
-
-// input layer weight gradient: dW0[i][f] += sum_b X[b][i] dZ1[b][f]
-__global__ void __launch_bounds__(256) mlp_in_grad_kernel(const float *__restrict__ X, const float *__restrict__ dZ1,
-                                                          float *grad, int n)
-{
-    const int f = threadIdx.x;
-    float acc[MLP_IN];
-#pragma unroll
-    for (int i = 0; i < MLP_IN; ++i) acc[i] = 0.f;
-    const int r0 = blockIdx.x * 128, r1 = min(n, r0 + 128);
-    for (int r = r0; r < r1; ++r) {
-        const float d = dZ1[(size_t)r * MLP_H + f];
-#pragma unroll
-        for (int i = 0; i < MLP_IN; ++i) acc[i] = fmaf(X[(size_t)r * MLP_XS + i], d, acc[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < MLP_IN; ++i) atomicAdd(grad + MLP_OFF_W0 + i * MLP_H + f, acc[i]);
-}
-
-__global__ void adam_kernel(float *P, const float *G, float *m, float *v, int n, float lr, float b1, float b2,
-                            float eps, float c1, float c2)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float g = G[i];
-    const float mi = b1 * m[i] + (1.f - b1) * g;
-    const float vi = b2 * v[i] + (1.f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    P[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-}
-
-// BF16 operand blocks of the hidden weights: Wt_j (rows out, K in) for the
-// forward GEMM, W_j (rows in, K out) for the backward-data GEMM, and Wq_j, Wt_j
-// as four contiguous 128 x 128 quarters (N half, K half) for the serving kernel
-struct WBlocks {
-    uint16_t *Wt[3], *W[3], *Wq[3];
-};
-
-__global__ void weights_to_blocks_kernel(const float *__restrict__ P, WBlocks wb)
-{
-    const int j = blockIdx.y + 1;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;  // out * 256 + in
-    if (e >= MLP_H * MLP_H) return;
-    const int out = e >> 8, in = e & 255;
-    const uint16_t b = f2bf(P[MLP_OFF_WT(j) + e]);
-    wb.Wt[j - 1][tc_core_offset(out, in, MLP_H) / 2] = b;
-    wb.W[j - 1][tc_core_offset(in, out, MLP_H) / 2] = b;
-    const int q = (out >> 7) * 2 + (in >> 7);
-    wb.Wq[j - 1][(size_t)q * 128 * 128 + tc_core_offset(out & 127, in & 127, 128) / 2] = b;
+    emit_tile(tile, st, rows_dst);
 }
 
 struct Mlp {
     int B = 0;  // batch capacity, multiple of 256
     int step = 0;
+    int nsm = 1;  // SMs of the device the buffers are on
     float *P = nullptr, *G = nullptr, *m = nullptr, *v = nullptr;
-    uint16_t *Wt[3] = {}, *W[3] = {}, *Wq[3] = {};
-    uint16_t *Hrows[3] = {}, *HT[3] = {};
-    float *H4 = nullptr;  // last hidden layer, FP32 row-major (training)
-    uint16_t *Gz[4] = {};
-    uint16_t *dZrows[3] = {}, *dZT[3] = {};  // index j-2 for dZ_j, j = 2..4
-    float *dZ1 = nullptr, *Y = nullptr, *loss = nullptr;
+    MlpBlocks blk = {};
+    MlpTrainBuf buf = {};
+    float *loss = nullptr;
     int *err = nullptr;
     std::vector<void *> allocs;  // every device allocation, freed with the object
     Mlp() = default;
@@ -482,17 +214,6 @@ bool mlp_alloc(Mlp &M, T **p, size_t count)
     return true;
 }
 
-WBlocks mlp_blocks(const Mlp &M)
-{
-    WBlocks b;
-    for (int j = 0; j < 3; ++j) {
-        b.Wt[j] = M.Wt[j];
-        b.W[j] = M.W[j];
-        b.Wq[j] = M.Wq[j];
-    }
-    return b;
-}
-
 void mlp_free(Mlp *M) { delete M; }
 
 template <class Epi>
@@ -507,33 +228,33 @@ cudaError_t gemm(const uint16_t *A, const uint16_t *Bop, int tiles, int K, int s
     return cudaGetLastError();
 }
 
-// Forward pass.  train: keep what the backward pass reads (transposed blocks,
-// gelu'(Z), the FP32 last hidden layer H4) and leave the output layer to
-// mlp_out_kernel; otherwise the output layer runs in the last epilogue -> Y.
-cudaError_t mlp_forward(Mlp &M, const float *X, int n, bool train, float *Y, cudaStream_t st)
+// Forward pass layer by layer; the output layer runs in the last epilogue -> Y.
+cudaError_t mlp_forward(Mlp &M, const float *X, int n, float *Y, cudaStream_t st)
 {
-    const int tiles = n / 128, nchunks = n / 256;
+    const int tiles = n / 128;
     cudaFuncSetAttribute(mlp_in_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * MLP_H * 2);
-    mlp_in_fwd_kernel<<<tiles, 256, 128 * MLP_H * 2, st>>>(X, M.P, M.Hrows[0], train ? M.HT[0] : nullptr,
-                                                            train ? M.Gz[0] : nullptr, nchunks);
+    mlp_in_fwd_kernel<<<tiles, 256, 128 * MLP_H * 2, st>>>(X, M.P, M.buf.H[0]);
     for (int j = 1; j <= 3; ++j) {
         EpiFwd e;
         e.bias = M.P + MLP_OFF_B(j);
-        e.rows_dst = j < 3 ? M.Hrows[j] : nullptr;
-        e.T_dst = train && j < 3 ? M.HT[j] : nullptr;
-        e.G_dst = train ? M.Gz[j] : nullptr;
-        e.h32_dst = train && j == 3 ? M.H4 : nullptr;
+        e.rows_dst = j < 3 ? M.buf.H[j] : nullptr;
         e.W4 = M.P + MLP_OFF_W4;
         e.b4 = M.P + MLP_OFF_B4;
-        e.Y = !train && j == 3 ? Y : nullptr;
-        e.nchunks = nchunks;
-        cudaError_t c = gemm(M.Hrows[j - 1], M.Wt[j - 1], tiles, MLP_H, 1, e, M.err, st);
+        e.Y = j == 3 ? Y : nullptr;
+        cudaError_t c = gemm(M.buf.H[j - 1], M.blk.Wt[j - 1], tiles, MLP_H, 1, e, M.err, st);
         if (c != cudaSuccess) return c;
     }
     return cudaGetLastError();
 }
 
-const size_t OUT_SMEM = 128 * MLP_H * 2 + MLP_H * MLP_OUT * 4 + 128 * 16;
+int device_sms()
+{
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1)
+        nsm = 1;
+    return nsm;
+}
 
 }  // namespace
 
@@ -546,17 +267,20 @@ int bldfm_surrogate_create(int32_t batch, uint64_t seed, void **handle)
         std::unique_ptr<Mlp> own(new Mlp());  // freed on every early return
         Mlp *M = own.get();
         M->B = batch;
+        M->nsm = device_sms();
         const size_t B = (size_t)batch;
         bool ok = mlp_alloc(*M, &M->P, MLP_NPARAM) && mlp_alloc(*M, &M->G, MLP_NPARAM) &&
                   mlp_alloc(*M, &M->m, MLP_NPARAM) && mlp_alloc(*M, &M->v, MLP_NPARAM) &&
-                  mlp_alloc(*M, &M->H4, B * MLP_H) && mlp_alloc(*M, &M->dZ1, B * MLP_H) &&
-                  mlp_alloc(*M, &M->Y, B * MLP_OUT) && mlp_alloc(*M, &M->loss, 1) && mlp_alloc(*M, &M->err, 1);
+                  mlp_alloc(*M, &M->loss, 1) && mlp_alloc(*M, &M->err, 1) &&
+                  mlp_alloc(*M, &M->buf.part_w, mlp_train_part_w(batch, M->nsm)) &&
+                  mlp_alloc(*M, &M->buf.part_o, mlp_train_part_o(batch, M->nsm)) &&
+                  mlp_alloc(*M, &M->buf.Xp, B * 32) && mlp_alloc(*M, &M->buf.D[3], B * MLP_H);
+        const size_t W = (size_t)MLP_H * MLP_H;
         for (int j = 0; j < 3 && ok; ++j)
-            ok = mlp_alloc(*M, &M->Wt[j], (size_t)MLP_H * MLP_H) && mlp_alloc(*M, &M->W[j], (size_t)MLP_H * MLP_H) &&
-                 mlp_alloc(*M, &M->Wq[j], (size_t)MLP_H * MLP_H) &&
-                 mlp_alloc(*M, &M->Hrows[j], B * MLP_H) && mlp_alloc(*M, &M->HT[j], B * MLP_H) &&
-                 mlp_alloc(*M, &M->dZrows[j], B * MLP_H) && mlp_alloc(*M, &M->dZT[j], B * MLP_H);
-        for (int j = 0; j < 4 && ok; ++j) ok = mlp_alloc(*M, &M->Gz[j], B * MLP_H);
+            ok = mlp_alloc(*M, &M->blk.Wf[j], W) && mlp_alloc(*M, &M->blk.Wb[j], W) &&
+                 mlp_alloc(*M, &M->blk.Wt[j], W) && mlp_alloc(*M, &M->blk.Wq[j], W) &&
+                 mlp_alloc(*M, &M->buf.H[j], B * MLP_H) && mlp_alloc(*M, &M->buf.D[j], B * MLP_H) &&
+                 mlp_alloc(*M, &M->buf.G[j], B * MLP_H);
         if (!ok) return BLDFM_ERR_CUDA;
         // He-scaled normal weights (Box-Muller on a 64-bit LCG), zero biases
         std::vector<float> p(MLP_NPARAM, 0.f);
@@ -575,8 +299,8 @@ int bldfm_surrogate_create(int32_t batch, uint64_t seed, void **handle)
         cudaMemset(M->v, 0, MLP_NPARAM * 4);
         cudaMemset(M->G, 0, MLP_NPARAM * 4);
         cudaMemset(M->err, 0, 4);
-        weights_to_blocks_kernel<<<dim3(MLP_H * MLP_H / 256, 3), 256>>>(M->P, mlp_blocks(*M));
-        if (cudaDeviceSynchronize() != cudaSuccess) return BLDFM_ERR_CUDA;
+        if (launch_mlp_blocks(M->P, M->blk, 0) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+            return BLDFM_ERR_CUDA;
         *handle = own.release();
         return BLDFM_OK;
     });
@@ -604,8 +328,8 @@ int bldfm_surrogate_params(void *handle, float *host_out, const float *host_in)
         return BLDFM_ERR_CUDA;
     if (host_in) {
         if (cudaMemcpy(M->P, host_in, MLP_NPARAM * 4, cudaMemcpyHostToDevice) != cudaSuccess) return BLDFM_ERR_CUDA;
-        weights_to_blocks_kernel<<<dim3(MLP_H * MLP_H / 256, 3), 256>>>(M->P, mlp_blocks(*M));
-        if (cudaDeviceSynchronize() != cudaSuccess) return BLDFM_ERR_CUDA;
+        if (launch_mlp_blocks(M->P, M->blk, 0) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+            return BLDFM_ERR_CUDA;
     }
     return BLDFM_OK;
 }
@@ -632,39 +356,25 @@ int bldfm_surrogate_train_step(void *handle, const float *X, const float *T, con
 {
     Mlp *M = (Mlp *)handle;
     if (!M || !X || !T || !w || n < 256 || n > M->B || n % 256 != 0) return BLDFM_ERR_ARG;
-    cudaStream_t st = (cudaStream_t)stream;
-    const int tiles = n / 128, nchunks = n / 256;
-    if (cudaMemsetAsync(M->G, 0, MLP_NPARAM * 4, st) != cudaSuccess) return BLDFM_ERR_CUDA;
-    if (cudaMemsetAsync(M->loss, 0, 4, st) != cudaSuccess) return BLDFM_ERR_CUDA;
-    if (mlp_forward(*M, X, n, true, nullptr, st) != cudaSuccess) return BLDFM_ERR_CUDA;
-    cudaFuncSetAttribute(mlp_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OUT_SMEM);
-    mlp_out_kernel<<<tiles, 128, OUT_SMEM, st>>>(M->H4, M->Gz[3], M->P, T, w, 1.0f / n, M->Y, M->G, M->loss,
-                                                 M->dZrows[2], M->dZT[2], nchunks, n);
-    // hidden layers, last to first: dW_j from dZ_{j+1}^T and H_j^T, dH_j from dZ_{j+1} and W_j
-    for (int j = 3; j >= 1; --j) {
-        EpiGrad eg;
-        eg.grad = M->G + MLP_OFF_WT(j);
-        const int splits = nchunks < 64 ? nchunks : 64;
-        if (gemm(M->dZT[j - 1], M->HT[j - 1], 2, n, splits, eg, M->err, st) != cudaSuccess) return BLDFM_ERR_CUDA;
-        EpiBwd eb;
-        eb.G = M->Gz[j - 1];
-        eb.rows_dst = j > 1 ? M->dZrows[j - 2] : nullptr;
-        eb.T_dst = j > 1 ? M->dZT[j - 2] : nullptr;
-        eb.rowmajor_f32 = j == 1 ? M->dZ1 : nullptr;
-        eb.dbias = M->G + (j > 1 ? MLP_OFF_B(j - 1) : MLP_OFF_B0);
-        eb.nchunks = nchunks;
-        if (gemm(M->dZrows[j - 1], M->W[j - 1], tiles, MLP_H, 1, eb, M->err, st) != cudaSuccess) return BLDFM_ERR_CUDA;
-    }
-    mlp_in_grad_kernel<<<tiles, 256, 0, st>>>(X, M->dZ1, M->G, n);
+    MlpAdam ad;
+    ad.P = M->P;
+    ad.G = M->G;
+    ad.m = M->m;
+    ad.v = M->v;
+    ad.loss = M->loss;
+    ad.lr = lr;
+    ad.b1 = 0.9f;
+    ad.b2 = 0.999f;
+    ad.eps = 1e-8f;
+    ad.c1 = ad.c2 = 1.f;
     if (lr != 0.f) {
         M->step += 1;
-        const float b1 = 0.9f, b2 = 0.999f;
-        const float c1 = 1.f / (1.f - powf(b1, (float)M->step)), c2 = 1.f / (1.f - powf(b2, (float)M->step));
-        adam_kernel<<<(MLP_NPARAM + 255) / 256, 256, 0, st>>>(M->P, M->G, M->m, M->v, MLP_NPARAM, lr, b1, b2, 1e-8f,
-                                                              c1, c2);
-        weights_to_blocks_kernel<<<dim3(MLP_H * MLP_H / 256, 3), 256, 0, st>>>(M->P, mlp_blocks(*M));
+        ad.c1 = 1.f / (1.f - powf(ad.b1, (float)M->step));
+        ad.c2 = 1.f / (1.f - powf(ad.b2, (float)M->step));
     }
-    return cudaGetLastError() == cudaSuccess ? BLDFM_OK : BLDFM_ERR_CUDA;
+    return launch_mlp_train(X, T, w, n, M->buf, M->blk, ad, M->err, M->nsm, (cudaStream_t)stream) == cudaSuccess
+               ? BLDFM_OK
+               : BLDFM_ERR_CUDA;
 }
 
 // Y [n][4] = MLP(X [n][8]), n % 256 == 0, device pointers (forward only: the
@@ -674,7 +384,7 @@ int bldfm_surrogate_forward(void *handle, const float *X, float *Y, int32_t n, v
     Mlp *M = (Mlp *)handle;
     if (!M || !X || !Y || n < 256 || n > M->B || n % 256 != 0) return BLDFM_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    if (mlp_forward(*M, X, n, false, Y, st) != cudaSuccess) return BLDFM_ERR_CUDA;
+    if (mlp_forward(*M, X, n, Y, st) != cudaSuccess) return BLDFM_ERR_CUDA;
     return BLDFM_OK;
 }
 
@@ -686,8 +396,8 @@ int mlp_serving_view(void *handle, MlpServing *out)
     if (!M || !out) return BLDFM_ERR_ARG;
     out->P = M->P;
     for (int j = 0; j < 3; ++j) {
-        out->Wt[j] = M->Wt[j];
-        out->Wq[j] = M->Wq[j];
+        out->Wt[j] = M->blk.Wt[j];
+        out->Wq[j] = M->blk.Wq[j];
     }
     return BLDFM_OK;
 }

@@ -112,6 +112,48 @@ __device__ __forceinline__ void tc_mma(uint32_t dtmem, uint64_t adesc, uint64_t 
         : "memory");
 }
 
+// The same issued by a whole converged warp: one elected lane issues it.  In
+// warp-uniform code the compiler keeps descriptors and loop state in uniform
+// registers, which the instruction reads; issued from a branch that only one
+// lane takes, every operand is first moved there, 200 to 270 clocks per MMA
+// where the MMA itself (128 x 256 x 16) takes 128.
+__device__ __forceinline__ void tc_mma_warp(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+// tc_commit by a whole converged warp (the lane that issued the MMAs)
+__device__ __forceinline__ void tc_commit_warp(uint64_t *bar)
+{
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+            (uint32_t)__cvta_generic_to_shared(bar))
+        : "memory");
+}
+
+// tc_expect_tx and one bulk copy of `bytes` (at most 32 KB) by a whole
+// converged warp
+__device__ __forceinline__ void tc_load_warp(void *dst, const void *src, uint32_t bytes, uint32_t expect, uint64_t *bar)
+{
+    asm volatile(
+        "{\n\t.reg .pred q, x;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.and.b32 x, %4, 0, q;\n\t"
+        "@x mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n\t"
+        "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(
+            tc_smem(dst)),
+        "l"(src), "r"(bytes), "r"(tc_smem(bar)), "r"(expect)
+        : "memory");
+}
+
 // D[tmem] (+)= A[tmem] * B[smem]^T: A (M x K, BF16) in tensor memory, one
 // lane per row and two K values per 32-bit column (K = 16 spans 8 columns)
 __device__ __forceinline__ void tc_mma_ts(uint32_t dtmem, uint32_t atmem, uint64_t bdesc, uint32_t idesc,
@@ -200,6 +242,21 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float *v)
         : "memory");
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 consecutive FP32 columns of this thread's TMEM lane
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, float *v)
+{
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // 64 consecutive FP32 columns: two loads in flight, one wait
