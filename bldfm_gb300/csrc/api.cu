@@ -648,7 +648,7 @@ int solve_impl(const bldfm_desc *d, const double *srf_dev, const double *z, cons
         } else if (!shoot) {
             // accurate FP64 mode: invariant imbedding, no libm values needed
             CK(cudaEventRecord(slt->ev, st));
-            CK(launch_riccati64(g, lv64, slot, ml->dev, q0, (double *)(w + L.scratch), Xp, Xq, err, dc.nsm, st));
+            CK(launch_riccati64(g, lv64, slot, ml->dev, q0, (double *)(w + L.scratch), Xp, Xq, dc.nsm, st));
             tmark(dc, st);  // 2: after the sweep
             if (!g.footprint) CK(launch_trapezoid64(g, lv64, slot, q0, p000, dcv, st));
         } else {

@@ -15,6 +15,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "common.h"
 #include "devmath.cuh"
 #include "fft_core.cuh"
@@ -27,9 +30,86 @@
 // ---------------------------------------------------------------------------
 // FP64 shooting sweep
 // ---------------------------------------------------------------------------
-// One thread per solved mode.  Writes per mode: top states (p1,q1,p2,q2) and
-// the same four states at every snapshot slot.
+// FP64 instructions of this GPU take 16 clocks per warp and SM as an FMA of
+// three registers and 19 as an addition or a multiplication (0.628 against
+// 0.529 T lanes/s, measured with register operands; an FMA with a constant or
+// uniform operand takes 19 too).  a + b = fma(a, 1, b) and a b = fma(a, b, -0)
+// round, and sign their zeros, exactly as the addition and the product do, so
+// the sweep issues nothing but FMAs, the 1 and the -0 in registers the
+// compiler cannot see through (read from shared memory).
+struct FmaArith {
+    double one, mz, two9;
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(b, -one, a); }
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, mz); }
+    __device__ __forceinline__ double2 cmul(double2 a, double2 b) const
+    {
+        return make_double2(__fma_rn(a.x, b.x, -mul(a.y, b.y)), __fma_rn(a.x, b.y, mul(a.y, b.x)));
+    }
+    // a b for a = -n
+    __device__ __forceinline__ double2 cmul_neg(double2 n, double2 b) const
+    {
+        return make_double2(__fma_rn(-n.x, b.x, mul(n.y, b.y)), __fma_rn(-n.x, b.y, -mul(n.y, b.x)));
+    }
+    __device__ __forceinline__ double2 cadd(double2 a, double2 b) const
+    {
+        return make_double2(add(a.x, b.x), add(a.y, b.y));
+    }
+};
+
+// both shooting states of one mode
+struct Shoot {
+    double2 p1, q1, p2, q2;
+};
+
+// Items of the paired sweep (NM = 2): the modes (kx, ky) and (kx, -ky) of a
+// column share T's real part and what follows from it (Re a, Re b, Re T dz and
+// the four products inside T): 62 FP64 instructions a mode and step instead of
+// 68.  In the mode list's order, column 0 holds its C0 rows from row 1 on,
+// columns 1 .. F every row, the columns after them one row each (even nly).
+struct SweepItems {
+    int C0, F, I, n;  // I items per full column: rows 0 .. nly / 2; n items in all
+};
+
+__host__ __device__ inline SweepItems sweep_items(int nlx, int nly)
+{
+    SweepItems s;
+    s.C0 = freq_max(nly) + (nly % 2 == 0 ? 1 : 0);
+    s.F = nlx / 2;
+    s.I = nly / 2 + 1;
+    s.n = s.C0 + s.F * s.I + (nly % 2 == 0 ? nlx - 1 - s.F : 0);
+    return s;
+}
+
+// column, row and list index of item i; its partner's list index or -1
+__device__ __forceinline__ void sweep_item(const SweepItems &s, int nly, int i, int &c, int &r, int64_t &m0,
+                                           int64_t &m1)
+{
+    m1 = -1;
+    if (i < s.C0) {
+        c = 0;
+        r = i + 1;
+        m0 = i;
+        return;
+    }
+    const int j = i - s.C0;
+    if (j < s.F * s.I) {
+        c = 1 + j / s.I;
+        r = j - (c - 1) * s.I;
+        const int64_t base = s.C0 + (int64_t)(c - 1) * nly;
+        m0 = base + r;
+        if (r > 0 && 2 * r != nly) m1 = base + nly - r;
+        return;
+    }
+    c = s.F + 1 + (j - s.F * s.I);
+    r = nly / 2;
+    m0 = s.C0 + (int64_t)s.F * nly + (j - s.F * s.I);
+}
+
+// NM modes per thread (2: the items above).  Writes per mode: top states
+// (p1,q1,p2,q2) and the same four states at every snapshot slot.
 //   snap layout: [(slot * 4 + j) * nsolved + m],  top layout: [j * nsolved + m]
+template <int NM>
 __global__ void __launch_bounds__(128) sweep64_kernel(SolveGeom g, const double *__restrict__ lvtab,
                                                       const int *__restrict__ slot_of_step,
                                                       const uint32_t *__restrict__ modes,
@@ -39,77 +119,92 @@ __global__ void __launch_bounds__(128) sweep64_kernel(SolveGeom g, const double 
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t bar;
+    __shared__ double s_one[4];
     double *s_lv = (double *)smem_raw;
     const int L = g.nz - 1;
     int *s_slot = (int *)(s_lv + (size_t)L * BLDFM_LV64);
+    if (threadIdx.x < 4) s_one[threadIdx.x] = threadIdx.x < 2 ? 1.0 : -0.0;
     if (L > 0) {
         if (!bulk_load_to_smem(s_lv, lvtab, (uint32_t)((size_t)L * BLDFM_LV64 * sizeof(double)), &bar, err))
             return;
     }
     for (int i = threadIdx.x; i < g.nz; i += blockDim.x) s_slot[i] = slot_of_step[i];
     __syncthreads();
+    const FmaArith F = {s_one[threadIdx.x & 1], s_one[2 + (threadIdx.x & 1)], 0.0};
 
     const int64_t ns = g.nsolved;
-    for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m < ns; m += (int64_t)gridDim.x * blockDim.x) {
+    const SweepItems si = sweep_items(g.nlx, g.nly);
+    const int64_t n = NM == 2 ? si.n : ns;
+    for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it < n; it += (int64_t)gridDim.x * blockDim.x) {
         int r, c;
-        bool paired;
-        unpack_mode(modes[m], r, c, paired);
+        int64_t m[2] = {it, -1};
+        if (NM == 2) {
+            sweep_item(si, g.nly, (int)it, c, r, m[0], m[1]);
+        } else {
+            bool paired;
+            unpack_mode(modes[it], r, c, paired);
+        }
         const double lx = wavenumber(freq_of_index(c, g.nlx), g.valx, g.lx_scale);
         const double ly = wavenumber(freq_of_index(r, g.nly), g.valy, g.ly_scale);
         const double lx2 = __dmul_rn(lx, lx), ly2 = __dmul_rn(ly, ly);
-        double2 p1 = make_double2(1.0, 0.0), q1 = make_double2(0.0, 0.0);
-        double2 p2 = make_double2(0.0, 0.0);
-        double2 q2 = q0spec ? q0spec[(size_t)c * g.nly + r] : make_double2(g.q0dc_fp, 0.0);
+        Shoot S[NM];
+#pragma unroll
+        for (int u = 0; u < NM; ++u) {
+            S[u].p1 = make_double2(1.0, 0.0);
+            S[u].q1 = S[u].p2 = make_double2(0.0, 0.0);
+            S[u].q2 = q0spec ? q0spec[(size_t)c * g.nly + (u == 0 || r == 0 ? r : g.nly - r)]
+                             : make_double2(g.q0dc_fp, 0.0);
+        }
+        auto store = [&](double2 *o, int u) {
+            o += m[u];
+            o[0] = S[u].p1;
+            o[ns] = S[u].q1;
+            o[2 * ns] = S[u].p2;
+            o[3 * ns] = S[u].q2;
+        };
         for (int i = 0; i < L; ++i) {
             const int s = s_slot[i];
             if (s >= 0) {
-                double2 *o = snap + (size_t)s * 4 * ns + m;
-                o[0] = p1;
-                o[ns] = q1;
-                o[2 * ns] = p2;
-                o[3 * ns] = q2;
+                store(snap + (size_t)s * 4 * ns, 0);
+                if (NM == 2 && m[NM - 1] >= 0) store(snap + (size_t)s * 4 * ns, NM - 1);
             }
             const double *lv = s_lv + (size_t)i * BLDFM_LV64;
-            // T = -(Kx Lx^2 + Ky Ly^2) - 1j u Lx - 1j v Ly
-            double2 T;
-            T.x = -__dadd_rn(__dmul_rn(lv[LV_KX], lx2), __dmul_rn(lv[LV_KY], ly2));
-            T.y = __dsub_rn(-__dmul_rn(lv[LV_U], lx), __dmul_rn(lv[LV_V], ly));
-            // a = d = 1 - 0.5 Kzinv T dz^2
-            double2 a;
-            a.x = __dsub_rn(1.0, __dmul_rn(__dmul_rn(lv[LV_S1], T.x), lv[LV_H2]));
-            a.y = __dsub_rn(0.0, __dmul_rn(__dmul_rn(lv[LV_S1], T.y), lv[LV_H2]));
-            // b = -Kzinv dz - 1/6 Kzinv^2 T dz^3
-            double2 b;
-            b.x = __dsub_rn(lv[LV_S3], __dmul_rn(__dmul_rn(lv[LV_S2], T.x), lv[LV_H3]));
-            b.y = __dsub_rn(0.0, __dmul_rn(__dmul_rn(lv[LV_S2], T.y), lv[LV_H3]));
-            // c = T dz - 1/6 Kzinv T^2 dz^3
-            const double2 T2 = np_cmul(T, T);
-            double2 cc;
-            cc.x = __dsub_rn(__dmul_rn(T.x, lv[LV_H]), __dmul_rn(__dmul_rn(lv[LV_S4], T2.x), lv[LV_H3]));
-            cc.y = __dsub_rn(__dmul_rn(T.y, lv[LV_H]), __dmul_rn(__dmul_rn(lv[LV_S4], T2.y), lv[LV_H3]));
-            const double2 np1 = np_cadd(np_cmul(a, p1), np_cmul(b, q1));
-            const double2 nq1 = np_cadd(np_cmul(cc, p1), np_cmul(a, q1));
-            const double2 np2 = np_cadd(np_cmul(a, p2), np_cmul(b, q2));
-            const double2 nq2 = np_cadd(np_cmul(cc, p2), np_cmul(a, q2));
-            p1 = np1;
-            q1 = nq1;
-            p2 = np2;
-            q2 = nq2;
-        }
-        {
-            const int s = s_slot[g.nz - 1];
-            if (s >= 0) {
-                double2 *o = snap + (size_t)s * 4 * ns + m;
-                o[0] = p1;
-                o[ns] = q1;
-                o[2 * ns] = p2;
-                o[3 * ns] = q2;
+            // T = -(Kx Lx^2 + Ky Ly^2) - 1j u Lx - 1j v Ly = -(tx + 1j ty)
+            const double tx = F.add(F.mul(lv[LV_KX], lx2), F.mul(lv[LV_KY], ly2));
+            const double ul = F.mul(lv[LV_U], lx), vl = F.mul(lv[LV_V], ly);
+            // real parts of a = d = 1 - 0.5 Kzinv T dz^2 and
+            // b = -Kzinv dz - 1/6 Kzinv^2 T dz^3; T dz
+            const double ax = F.add(F.mul(F.mul(lv[LV_S1], tx), lv[LV_H2]), F.one);
+            const double bx = F.add(F.mul(F.mul(lv[LV_S2], tx), lv[LV_H3]), lv[LV_S3]);
+            const double txh = F.mul(tx, lv[LV_H]);
+#pragma unroll
+            for (int u = 0; u < NM; ++u) {
+                const double ty = u == 0 ? F.add(ul, vl) : F.sub(ul, vl);
+                const double2 a = make_double2(ax, F.mul(F.mul(lv[LV_S1], ty), lv[LV_H2]));
+                const double2 b = make_double2(bx, F.mul(F.mul(lv[LV_S2], ty), lv[LV_H3]));
+                // c = T dz - 1/6 Kzinv T^2 dz^3, negated
+                const double2 T2 = F.cmul(make_double2(tx, ty), make_double2(tx, ty));
+                const double2 cn =
+                    make_double2(F.add(F.mul(F.mul(lv[LV_S4], T2.x), lv[LV_H3]), txh),
+                                 F.add(F.mul(F.mul(lv[LV_S4], T2.y), lv[LV_H3]), F.mul(ty, lv[LV_H])));
+                Shoot &x = S[u];
+                const double2 np1 = F.cadd(F.cmul(a, x.p1), F.cmul(b, x.q1));
+                const double2 nq1 = F.cadd(F.cmul_neg(cn, x.p1), F.cmul(a, x.q1));
+                const double2 np2 = F.cadd(F.cmul(a, x.p2), F.cmul(b, x.q2));
+                const double2 nq2 = F.cadd(F.cmul_neg(cn, x.p2), F.cmul(a, x.q2));
+                x.p1 = np1;
+                x.q1 = nq1;
+                x.p2 = np2;
+                x.q2 = nq2;
             }
         }
-        top[m] = p1;
-        top[ns + m] = q1;
-        top[2 * ns + m] = p2;
-        top[3 * ns + m] = q2;
+        const int s = s_slot[g.nz - 1];
+#pragma unroll
+        for (int u = 0; u < NM; ++u) {
+            if (u > 0 && m[u] < 0) break;
+            if (s >= 0) store(snap + (size_t)s * 4 * ns, u);
+            store(top, u);
+        }
     }
 }
 
@@ -339,205 +434,283 @@ __device__ __forceinline__ double2 dc_mul(double2 a, double2 b)
     return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
 }
 
-// 1/x for a positive normal x: the approximate hardware reciprocal refined by
-// two Newton-Raphson steps for f(y) = 1/y - x (y <- y + y (1 - x y)), each of
-// which doubles the number of correct bits, to within an ulp or two of the
-// rounded quotient.  Faster than the IEEE division, whose exact rounding the
-// accurate FP64 mode does not need.
-__device__ __forceinline__ double rcp_newton(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double e = fma(-x, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-x, y, 1.0);
-    return fma(y, e, y);
-}
-
-// Per-level products of the accurate FP64 sweep's step coefficients
-// (A = S1 H2, B1 = S2 H3, C1 = S4 H3), formed once per CTA in shared memory
-#define RICC64_K 3
+// Accurate FP64 sweep: invariant imbedding in its homogeneous form.  The ratio
+// R_i = p_i / q_i of the decaying solution is N_i / D_i with
+//   N <- a N - b D,   D <- a D - c N
+// (16 FMAs a step where the update of R with its reciprocal takes 22), and the
+// flux factors telescope: q_j / q_0 = (D_j / D_0) prod_{i<j} det_i with
+// det_i = a^2 - b c.  With w = a - 1 the step's coefficients are
+//   a = 1 + w,  b = B0 - (B0 / 3) w,  c = g (w + w^2 / 3),  g = 2 / B0,
+//   det = 1 + w^2 + (2/9) w^3,
+// w = (A Kx lx^2 + A Ky ly^2) + i (A u lx + A v ly), A = dz^2 / (2 Kz),
+// B0 = -dz / Kz.  The FP64 pipe bounds it (FmaArith above): 27 instructions a
+// mode and step above the highest output level and 36.5 below it for a pair of
+// modes (kx, +-ky) per thread, 30 and 40 alone; the ratio form took 38 and 46,
+// a third of them additions and multiplications.  States and determinant are
+// rescaled by powers of two every 4 steps (integer arithmetic on the exponent).
+enum { RT_AKX, RT_AKY, RT_AU, RT_AV, RT_B0, RT_B1, RT_G, RT_G3, RT_N };
 #define RICC64_SMEM (200 * 1024)  // dynamic shared memory the kernel is set up for
 
-template <bool SINGLE>
+// exponent of the largest of n values (0 for zeros and non-finite values)
+__device__ __forceinline__ int top_exponent(const double *v, int n)
+{
+    int e = 0;
+#pragma unroll
+    for (int k = 0; k < n; ++k) e = max(e, (__double2hiint(v[k]) >> 20) & 0x7ff);
+    return e == 0 || e == 0x7ff ? 0 : e - 1023;
+}
+// v 2^-e (values outside the normal range, before or after, become zero)
+__device__ __forceinline__ double scale_down(double v, int e)
+{
+    const int hi = __double2hiint(v), x = (hi >> 20) & 0x7ff;
+    if (x == 0x7ff) return v;
+    return x == 0 || x - e <= 0 ? 0.0 : __hiloint2double(hi - e * (1 << 20), __double2loint(v));
+}
+
+struct RiccState {
+    double n[4];  // N, D (re, im)
+    double2 P;    // product of det_i below the highest output level
+    int E, EP;    // their powers of two
+};
+
+template <bool SINGLE, int NM>
 __global__ void __launch_bounds__(128) riccati64_kernel(SolveGeom g, const double *__restrict__ lvtab,
                                                         const int *__restrict__ slot_of_step,
                                                         const uint32_t *__restrict__ modes,
                                                         const double2 *__restrict__ q0spec,
                                                         double *__restrict__ scratch, double2 *__restrict__ Xp,
-                                                        double2 *__restrict__ Xq, int *err, bool kprod)
+                                                        double2 *__restrict__ Xq)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ uint64_t bar;
-    double *s_lv = (double *)smem_raw;
+    __shared__ double s_one[6];
+    double *s_rt = (double *)smem_raw;
     const int L = g.nz - 1;
-    int *s_slot = (int *)(s_lv + (size_t)L * BLDFM_LV64);
-    if (L > 0) {
-        if (!bulk_load_to_smem(s_lv, lvtab, (uint32_t)((size_t)L * BLDFM_LV64 * sizeof(double)), &bar, err))
-            return;
+    int *s_slot = (int *)(s_rt + (size_t)L * RT_N);
+    if (threadIdx.x < 6) s_one[threadIdx.x] = threadIdx.x < 2 ? 1.0 : threadIdx.x < 4 ? -0.0 : 2.0 / 9.0;
+    for (int i = threadIdx.x; i < L; i += blockDim.x) {
+        const double *lv = lvtab + (size_t)i * BLDFM_LV64;
+        double *o = s_rt + (size_t)i * RT_N;
+        const double A = lv[LV_S1] * lv[LV_H2], B0 = lv[LV_S3], G = 2.0 / B0;
+        o[RT_AKX] = A * lv[LV_KX];
+        o[RT_AKY] = A * lv[LV_KY];
+        o[RT_AU] = A * lv[LV_U];
+        o[RT_AV] = A * lv[LV_V];
+        o[RT_B0] = B0;
+        o[RT_B1] = -B0 / 3.0;
+        o[RT_G] = G;
+        o[RT_G3] = G / 3.0;
     }
     for (int i = threadIdx.x; i < g.nz; i += blockDim.x) s_slot[i] = slot_of_step[i];
-    // after the slot map, 8-byte aligned
-    double *s_k = (double *)(smem_raw + ((((size_t)L * BLDFM_LV64 * sizeof(double) + (size_t)g.nz * sizeof(int)) + 7) &
-                                         ~(size_t)7));
     __syncthreads();
-    for (int i = threadIdx.x; kprod && i < L; i += blockDim.x) {
-        const double *lv = s_lv + (size_t)i * BLDFM_LV64;
-        s_k[RICC64_K * i] = lv[LV_S1] * lv[LV_H2];
-        s_k[RICC64_K * i + 1] = lv[LV_S2] * lv[LV_H3];
-        s_k[RICC64_K * i + 2] = lv[LV_S4] * lv[LV_H3];
-    }
-    __syncthreads();
+    const FmaArith F = {s_one[threadIdx.x & 1], s_one[2 + (threadIdx.x & 1)], s_one[4 + (threadIdx.x & 1)]};
     const int jmax = g.jmax;
     const int64_t ns = g.nsolved;
-    for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m < ns; m += (int64_t)gridDim.x * blockDim.x) {
+    const SweepItems si = sweep_items(g.nlx, g.nly);
+    const int64_t n = NM == 2 ? si.n : ns;
+    for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it < n; it += (int64_t)gridDim.x * blockDim.x) {
         int r, c;
-        bool paired;
-        unpack_mode(modes[m], r, c, paired);
+        int64_t m[2] = {it, -1};
+        if (NM == 2) {
+            sweep_item(si, g.nly, (int)it, c, r, m[0], m[1]);
+        } else {
+            bool paired;
+            unpack_mode(modes[it], r, c, paired);
+        }
         const int kx = freq_of_index(c, g.nlx), ky = freq_of_index(r, g.nly);
         const double lx = wavenumber(kx, g.valx, g.lx_scale), ly = wavenumber(ky, g.valy, g.ly_scale);
         const double lx2 = lx * lx, ly2 = ly * ly;
-        const double2 eg = csqrt_d(make_double2(fma(g.kxk_top, lx2, g.kyk_top * ly2), fma(g.uk_top, lx, g.vk_top * ly)));
-        const double2 ke = make_double2(g.kz_top * eg.x, g.kz_top * eg.y);
-        const double kn = 1.0 / fma(ke.x, ke.x, ke.y * ke.y);
-        double2 R = make_double2(ke.x * kn, -ke.y * kn);
-        double2 Q = make_double2(1.0, 0.0), Rj = R;
-        int E = 0;
-        auto coef = [&](int i, double2 &a, double2 &b, double2 &cc) {
-            const double *lv = s_lv + (size_t)i * BLDFM_LV64;
-            const double Tr = -fma(lv[LV_KX], lx2, lv[LV_KY] * ly2);
-            const double Ti = -fma(lv[LV_U], lx, lv[LV_V] * ly);
-            double A, B1, C1;
-            if (kprod) {  // the same for every thread of the launch
-                const double *k = s_k + RICC64_K * i;
-                A = k[0];
-                B1 = k[1];
-                C1 = k[2];
-            } else {
-                A = lv[LV_S1] * lv[LV_H2];
-                B1 = lv[LV_S2] * lv[LV_H3];
-                C1 = lv[LV_S4] * lv[LV_H3];
+        RiccState S[NM];
+#pragma unroll
+        for (int u = 0; u < NM; ++u) {
+            const double l = u == 0 ? ly : -ly;
+            const double2 eg =
+                csqrt_d(make_double2(fma(g.kxk_top, lx2, g.kyk_top * ly2), fma(g.uk_top, lx, g.vk_top * l)));
+            const double2 ke = make_double2(g.kz_top * eg.x, g.kz_top * eg.y);
+            const double kn = 1.0 / fma(ke.x, ke.x, ke.y * ke.y);
+            S[u].n[0] = ke.x * kn;
+            S[u].n[1] = -ke.y * kn;
+            S[u].n[2] = 1.0;
+            S[u].n[3] = 0.0;
+            S[u].P = make_double2(1.0, 0.0);
+            S[u].E = S[u].EP = 0;
+        }
+        // one step down; DET: with the determinant
+        auto step = [&](int i, auto det) {
+            constexpr bool DET = decltype(det)::value;
+            const double *t = s_rt + (size_t)i * RT_N;
+            const double wr = __fma_rn(t[RT_AKX], lx2, F.mul(t[RT_AKY], ly2));
+            const double ul = F.mul(t[RT_AU], lx), vl = F.mul(t[RT_AV], ly);
+            const double ar = F.add(wr, F.one), br = __fma_rn(t[RT_B1], wr, t[RT_B0]), gr = F.mul(t[RT_G], wr),
+                         w2 = F.mul(wr, wr), w9 = DET ? __fma_rn(F.two9, wr, F.one) : 0.0;
+#pragma unroll
+            for (int u = 0; u < NM; ++u) {
+                const double wi = u == 0 ? F.add(ul, vl) : F.sub(ul, vl);
+                const double bi = F.mul(t[RT_B1], wi);
+                const double sr = __fma_rn(-wi, wi, w2), h = F.mul(wr, wi);  // w^2 = sr + 2 i h
+                const double cr = __fma_rn(t[RT_G3], sr, gr);
+                const double h2 = F.add(h, h);
+                const double ci = __fma_rn(t[RT_G3], h2, F.mul(t[RT_G], wi));
+                double *v = S[u].n;
+                const double Nr = v[0], Ni = v[1], Dr = v[2], Di = v[3];
+                v[0] = __fma_rn(ar, Nr, __fma_rn(-wi, Ni, __fma_rn(-br, Dr, F.mul(bi, Di))));
+                v[1] = __fma_rn(ar, Ni, __fma_rn(wi, Nr, __fma_rn(-br, Di, -F.mul(bi, Dr))));
+                v[2] = __fma_rn(ar, Dr, __fma_rn(-wi, Di, __fma_rn(-cr, Nr, F.mul(ci, Ni))));
+                v[3] = __fma_rn(ar, Di, __fma_rn(wi, Dr, __fma_rn(-cr, Ni, -F.mul(ci, Nr))));
+                if (DET) {
+                    // det - 1 = w^2 (1 + (2/9) w)
+                    const double wi9 = F.mul(F.two9, wi);
+                    const double er = __fma_rn(sr, w9, -F.mul(h2, wi9)), ei = __fma_rn(sr, wi9, F.mul(h2, w9));
+                    const double2 P = S[u].P;
+                    S[u].P.x = __fma_rn(P.x, er, __fma_rn(-P.y, ei, P.x));
+                    S[u].P.y = __fma_rn(P.x, ei, __fma_rn(P.y, er, P.y));
+                }
             }
-            a = make_double2(fma(-A, Tr, 1.0), -A * Ti);
-            b = make_double2(fma(-B1, Tr, lv[LV_S3]), -B1 * Ti);
-            const double t2r = fma(Tr, Tr, -Ti * Ti), t2i = 2.0 * Tr * Ti;
-            cc = make_double2(fma(-C1, t2r, lv[LV_H] * Tr), fma(-C1, t2i, lv[LV_H] * Ti));
         };
-        auto step = [&](const double2 a, const double2 b, const double2 cc) {
-            const double2 cR = dc_mul(cc, R);
-            const double2 D = make_double2(a.x - cR.x, a.y - cR.y);
-            const double2 N = make_double2(fma(a.x, R.x, fma(-a.y, R.y, -b.x)), fma(a.x, R.y, fma(a.y, R.x, -b.y)));
-            const double dinv = rcp_newton(fma(D.x, D.x, D.y * D.y));
-            R = make_double2(fma(N.x, D.x, N.y * D.y) * dinv, fma(N.y, D.x, -N.x * D.y) * dinv);
+        auto rescale = [&](bool det) {
+#pragma unroll
+            for (int u = 0; u < NM; ++u) {
+                const int e = top_exponent(S[u].n, 4);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) S[u].n[k] = scale_down(S[u].n[k], e);
+                S[u].E += e;
+                if (det) {
+                    const double pv[2] = {S[u].P.x, S[u].P.y};
+                    const int ep = top_exponent(pv, 2);
+                    S[u].P = make_double2(scale_down(pv[0], ep), scale_down(pv[1], ep));
+                    S[u].EP += ep;
+                }
+            }
         };
         int i = L - 1;
         for (; i >= jmax; --i) {
-            double2 a, b, cc;
-            coef(i, a, b, cc);
-            step(a, b, cc);
+            step(i, std::false_type());
+            if ((i & 3) == 0) rescale(false);
         }
-        Rj = R;
-        if (!SINGLE) {
-            const int s = s_slot[jmax];
-            double *o = scratch + (size_t)s * 5 * ns + m;
-            o[0] = R.x;
-            o[ns] = R.y;
-            o[2 * ns] = 1.0;
-            o[3 * ns] = 0.0;
-            o[4 * ns] = 0.0;
-        }
+        RiccState J[NM];  // the states at the highest output level
+#pragma unroll
+        for (int u = 0; u < NM; ++u) J[u] = S[u];
+        // scratch of an output slot: (N, D) / P and its power of two
+        auto keep = [&](int s) {
+#pragma unroll
+            for (int u = 0; u < NM; ++u) {
+                if (m[u] < 0) continue;
+                double *o = scratch + (size_t)s * 5 * ns + m[u];
+                const double2 P = S[u].P;
+                const double pn = 1.0 / fma(P.x, P.x, P.y * P.y);
+                const double2 inv = make_double2(P.x * pn, -P.y * pn);
+                const double2 N = dc_mul(make_double2(S[u].n[0], S[u].n[1]), inv),
+                              D = dc_mul(make_double2(S[u].n[2], S[u].n[3]), inv);
+                o[0] = N.x;
+                o[ns] = N.y;
+                o[2 * ns] = D.x;
+                o[3 * ns] = D.y;
+                o[4 * ns] = (double)(S[u].E - S[u].EP);
+            }
+        };
+        if (!SINGLE) keep(s_slot[jmax]);
         for (; i >= 0; --i) {
-            double2 a, b, cc;
-            coef(i, a, b, cc);
-            step(a, b, cc);
-            Q = dc_mul(Q, make_double2(fma(cc.x, R.x, fma(-cc.y, R.y, a.x)), fma(cc.x, R.y, fma(cc.y, R.x, a.y))));
-            if ((i & 15) == 0) {
-                int e;
-                frexp(fmax(fabs(Q.x), fabs(Q.y)), &e);
-                Q.x = ldexp(Q.x, -e);
-                Q.y = ldexp(Q.y, -e);
-                E += e;
-            }
-            if (!SINGLE) {
-                const int s = s_slot[i];
-                if (s >= 0) {
-                    double *o = scratch + (size_t)s * 5 * ns + m;
-                    o[0] = R.x;
-                    o[ns] = R.y;
-                    o[2 * ns] = Q.x;
-                    o[3 * ns] = Q.y;
-                    o[4 * ns] = (double)E;
-                }
-            }
+            step(i, std::true_type());
+            if ((i & 3) == 0) rescale(true);
+            if (!SINGLE && s_slot[i] >= 0) keep(s_slot[i]);
         }
-        const double2 q0 = q0spec ? q0spec[(size_t)c * g.nly + r] : make_double2(g.q0dc_fp, 0.0);
-        double2 sh = make_double2(1.0, 0.0);
-        if (g.do_shift) {
-            const double th = lx * g.sx + ly * g.sy;
-            double sn, cs;
-            sincos(th, &sn, &cs);
-            sh = make_double2(cs, sn);
-        }
-        const int rm = paired ? index_of_freq(-ky, g.nly) : 0;
-        const int cm = paired ? index_of_freq(-kx, g.nlx) : 0;
-        for (int s = 0; s < (SINGLE ? 1 : g.nsnap); ++s) {
-            double2 ratio;
-            if (SINGLE) {
-                ratio = make_double2(ldexp(Q.x, E), ldexp(Q.y, E));
-            } else {
-                const double *o = scratch + (size_t)s * 5 * ns + m;
-                Rj = make_double2(o[0], o[ns]);
-                const double2 Qj = make_double2(o[2 * ns], o[3 * ns]);
-                const int Ej = (int)o[4 * ns];
-                const double qn = fma(Qj.x, Qj.x, Qj.y * Qj.y);
-                ratio = make_double2(0.0, 0.0);
-                if (qn > 0.0) {
-                    const double scl = ldexp(1.0 / qn, E - Ej);
-                    ratio = make_double2(fma(Q.x, Qj.x, Q.y * Qj.y) * scl, fma(Q.y, Qj.x, -Q.x * Qj.y) * scl);
-                }
-            }
-            double2 q = dc_mul(q0, ratio);
-            double2 p = dc_mul(Rj, q);
-            if (g.precision == 0) {
-                p = round_c64(p);
-                q = round_c64(q);
-            }
+#pragma unroll
+        for (int u = 0; u < NM; ++u) {
+            if (m[u] < 0) continue;
+            const int ru = u == 0 || r == 0 ? r : g.nly - r;
+            const int kyu = u == 0 ? ky : -ky;
+            const double lyu = u == 0 ? ly : -ly;
+            const double2 q0 = q0spec ? q0spec[(size_t)c * g.nly + ru] : make_double2(g.q0dc_fp, 0.0);
+            double2 sh = make_double2(1.0, 0.0);
             if (g.do_shift) {
-                p = dc_mul(p, sh);
-                q = dc_mul(q, sh);
+                const double th = lx * g.sx + lyu * g.sy;
+                double sn, cs;
+                sincos(th, &sn, &cs);
+                sh = make_double2(cs, sn);
             }
-            Xp[spec_idx(g, s, r, c)] = p;
-            Xq[spec_idx(g, s, r, c)] = q;
-            if (paired) {
-                Xp[spec_idx(g, s, rm, cm)] = make_double2(p.x, -p.y);
-                Xq[spec_idx(g, s, rm, cm)] = make_double2(q.x, -q.y);
+            // q0 P / D_0
+            const double2 D0 = make_double2(S[u].n[2], S[u].n[3]);
+            const double dn = 1.0 / fma(D0.x, D0.x, D0.y * D0.y);
+            const double2 G = dc_mul(q0, dc_mul(S[u].P, make_double2(D0.x * dn, -D0.y * dn)));
+            const int e0 = S[u].EP - S[u].E;
+            // the mirror of the mode, where it lies in the mode range
+            const bool paired = -kx >= freq_min(g.nlx) && -kx <= freq_max(g.nlx) && -kyu >= freq_min(g.nly) &&
+                                -kyu <= freq_max(g.nly);
+            const int rm = paired ? index_of_freq(-kyu, g.nly) : 0;
+            const int cm = paired ? index_of_freq(-kx, g.nlx) : 0;
+            for (int s = 0; s < (SINGLE ? 1 : g.nsnap); ++s) {
+                double2 N, D;
+                int e = e0;
+                if (SINGLE) {
+                    N = make_double2(J[u].n[0], J[u].n[1]);
+                    D = make_double2(J[u].n[2], J[u].n[3]);
+                    e += J[u].E;
+                } else {
+                    const double *o = scratch + (size_t)s * 5 * ns + m[u];
+                    N = make_double2(o[0], o[ns]);
+                    D = make_double2(o[2 * ns], o[3 * ns]);
+                    e += (int)o[4 * ns];
+                }
+                double2 q = dc_mul(D, G), p = dc_mul(N, G);
+                q = make_double2(ldexp(q.x, e), ldexp(q.y, e));
+                p = make_double2(ldexp(p.x, e), ldexp(p.y, e));
+                if (g.precision == 0) {
+                    p = round_c64(p);
+                    q = round_c64(q);
+                }
+                if (g.do_shift) {
+                    p = dc_mul(p, sh);
+                    q = dc_mul(q, sh);
+                }
+                Xp[spec_idx(g, s, ru, c)] = p;
+                Xq[spec_idx(g, s, ru, c)] = q;
+                if (paired) {
+                    Xp[spec_idx(g, s, rm, cm)] = make_double2(p.x, -p.y);
+                    Xq[spec_idx(g, s, rm, cm)] = make_double2(q.x, -q.y);
+                }
             }
         }
     }
 }
 
+// Modes per thread and threads per block of the FP64 sweeps.  The pipe passes
+// one instruction per 16 clocks and SM, whatever its warps, so a launch takes
+// (warps of the fullest SM) x (instructions of a warp): one1 for a warp of
+// single modes, one2 of pairs.  Pairs issue fewer in all but come in coarser
+// units, and reach 95% of the pipe's rate (single modes 99%).  Small blocks
+// spread a small solve evenly (256^2 modes: 772 us in blocks of one warp, 877
+// in blocks of four), larger ones where the level table leaves room for few.
+struct Sweep64Launch {
+    bool pairs;
+    int threads;
+    unsigned blocks;
+};
+
+static Sweep64Launch sweep64_launch(const SolveGeom &g, size_t smem, int nsm, double one1, double one2)
+{
+    const int64_t n2 = sweep_items(g.nlx, g.nly).n;
+    auto units = [&](int64_t n) { return (double)(((n + 31) / 32 + nsm - 1) / nsm); };
+    Sweep64Launch l;
+    l.pairs = units(n2) * one2 < 0.95 * units(g.nsolved) * one1;
+    const int64_t n = l.pairs ? n2 : g.nsolved;
+    const int fit = (int)((227 * 1024) / (smem + 1024));  // blocks per SM
+    l.threads = fit >= 8 ? 32 : fit >= 4 ? 64 : 128;
+    int64_t b = (n + l.threads - 1) / l.threads;
+    l.blocks = (unsigned)std::min<int64_t>(std::max<int64_t>(b, 1), 256LL * nsm);
+    return l;
+}
+
 cudaError_t launch_riccati64(const SolveGeom &g, const double *lvtab, const int *slot, const uint32_t *modes,
-                             const double2 *q0spec, double *scratch, double2 *Xp, double2 *Xq, int *err, int nsm,
-                             cudaStream_t st)
+                             const double2 *q0spec, double *scratch, double2 *Xp, double2 *Xq, int nsm, cudaStream_t st)
 {
     if (g.nsnap < 1 || g.nsolved == 0) return cudaSuccess;
-    // level table, slot map, then (8-byte aligned) the per-level products
-    // when they fit in the shared memory the kernel is set up for
-    const size_t base = (((size_t)(g.nz - 1) * BLDFM_LV64 * sizeof(double) + (size_t)g.nz * sizeof(int) + 7) &
-                         ~(size_t)7) +
-                        16;
-    const size_t withk = base + (size_t)(g.nz - 1) * RICC64_K * sizeof(double);
-    const bool kprod = withk <= RICC64_SMEM;
-    const size_t smem = kprod ? withk : base;
-    const int threads = 128;
-    int64_t blocks = (g.nsolved + threads - 1) / threads;
-    if (blocks > 64LL * nsm) blocks = 64LL * nsm;
+    const size_t smem = (size_t)(g.nz - 1) * RT_N * sizeof(double) + (size_t)g.nz * sizeof(int) + 16;
+    const double above = g.nz - 1 - g.jmax, below = g.jmax;
+    const Sweep64Launch l = sweep64_launch(g, smem, nsm, above * 30 + below * 40, above * 54 + below * 73);
+    auto run = [&](auto k) { k<<<l.blocks, l.threads, smem, st>>>(g, lvtab, slot, modes, q0spec, scratch, Xp, Xq); };
     if (g.nsnap == 1)
-        riccati64_kernel<true><<<(unsigned)blocks, threads, smem, st>>>(g, lvtab, slot, modes, q0spec, scratch, Xp,
-                                                                        Xq, err, kprod);
+        l.pairs ? run(riccati64_kernel<true, 2>) : run(riccati64_kernel<true, 1>);
     else
-        riccati64_kernel<false><<<(unsigned)blocks, threads, smem, st>>>(g, lvtab, slot, modes, q0spec, scratch, Xp,
-                                                                         Xq, err, kprod);
+        l.pairs ? run(riccati64_kernel<false, 2>) : run(riccati64_kernel<false, 1>);
     return LAUNCH_CHECK();
 }
 
@@ -694,13 +867,15 @@ cudaError_t launch_sweep64(const SolveGeom &g, const double *lvtab, const int *s
     const int L = g.nz - 1;
     const size_t smem = (size_t)L * BLDFM_LV64 * sizeof(double) + (size_t)g.nz * sizeof(int) + 16;
     static uint64_t attr = 0;
-    if (first_on_device(attr))
-        cudaFuncSetAttribute(sweep64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    const int threads = 128;
-    int64_t blocks = (g.nsolved + threads - 1) / threads;
-    if (blocks < 1) blocks = 1;
-    if (blocks > 64LL * nsm) blocks = 64LL * nsm;
-    sweep64_kernel<<<(unsigned)blocks, threads, smem, st>>>(g, lvtab, slot, modes, q0spec, snap, top, err);
+    if (first_on_device(attr)) {
+        cudaFuncSetAttribute(sweep64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(sweep64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    }
+    const Sweep64Launch l = sweep64_launch(g, smem, nsm, 68, 124);
+    if (l.pairs)
+        sweep64_kernel<2><<<l.blocks, l.threads, smem, st>>>(g, lvtab, slot, modes, q0spec, snap, top, err);
+    else
+        sweep64_kernel<1><<<l.blocks, l.threads, smem, st>>>(g, lvtab, slot, modes, q0spec, snap, top, err);
     return LAUNCH_CHECK();
 }
 
@@ -978,9 +1153,12 @@ void prepare_kernel_attributes()
 {
     set_fft_smem_attr<double>();
     set_fft_smem_attr<float>();
-    cudaFuncSetAttribute(sweep64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(riccati64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RICC64_SMEM);
-    cudaFuncSetAttribute(riccati64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RICC64_SMEM);
+    cudaFuncSetAttribute(sweep64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(sweep64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(riccati64_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, RICC64_SMEM);
+    cudaFuncSetAttribute(riccati64_kernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, RICC64_SMEM);
+    cudaFuncSetAttribute(riccati64_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, RICC64_SMEM);
+    cudaFuncSetAttribute(riccati64_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, RICC64_SMEM);
     cudaFuncSetAttribute(riccati32_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(riccati32_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(riccati32_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);

@@ -46,5 +46,5 @@ cudaError_t launch_nonfinite(const double *a, const double *b, int64_t n, int *f
 cudaError_t run_fma_peak(int kind, int nsm, cudaStream_t st, double *flops_per_s);
 void prepare_kernel_attributes();
 cudaError_t launch_riccati64(const SolveGeom &g, const double *lvtab, const int *slot, const uint32_t *modes,
-                             const double2 *q0spec, double *scratch, double2 *Xp, double2 *Xq, int *err, int nsm,
+                             const double2 *q0spec, double *scratch, double2 *Xp, double2 *Xq, int nsm,
                              cudaStream_t st);

@@ -70,6 +70,47 @@ __device__ __forceinline__ bool tc_mbar_wait(uint64_t *bar, uint32_t parity)
     return false;
 }
 
+// Bounded wait for an event that is near: polls first (a suspended wait takes
+// about 2 us to return, longer than the copy or MMA it waits for), then
+// suspends as tc_mbar_wait does.
+__device__ __forceinline__ bool tc_poll_wait(uint64_t *bar, uint32_t parity)
+{
+    const uint32_t b = tc_smem(bar);
+    for (int it = 0; it < 4096; ++it) {
+        uint32_t d;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(d)
+            : "r"(b), "r"(parity)
+            : "memory");
+        if (d) return true;
+    }
+    return tc_mbar_wait(bar, parity);
+}
+
+// named barrier of n threads
+__device__ __forceinline__ void tc_bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+// barrier that returns the conjunction of the threads' flags
+__device__ __forceinline__ bool tc_bar_and(int id, int n, bool f)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)f), "r"(id), "r"(n)
+        : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void tc_arrive(uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(bar)) : "memory");
+}
+
 __device__ __forceinline__ void tc_expect_tx(uint64_t *bar, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(bar)), "r"(bytes) : "memory");

@@ -76,26 +76,6 @@ __device__ __forceinline__ float4 load_row4(const float *__restrict__ p, bool al
     return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
 }
 
-// Bounded wait for an event that is near: polls first (a suspended wait takes
-// about 2 us to return, longer than the copy or MMA it waits for), then
-// suspends as tc_mbar_wait does.
-__device__ __forceinline__ bool ctl_wait(uint64_t *bar, uint32_t parity)
-{
-    const uint32_t b = tc_smem(bar);
-    for (int it = 0; it < 4096; ++it) {
-        uint32_t d;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(d)
-            : "r"(b), "r"(parity)
-            : "memory");
-        if (d) return true;
-    }
-    return tc_mbar_wait(bar, parity);
-}
-
 __device__ __forceinline__ void lds8(float *v, const float *p)
 {
     const float4 a = *(const float4 *)p, b = *(const float4 *)(p + 4);
@@ -129,26 +109,6 @@ const int OFF_BIAS = OFF_STG + 4 * STG;
 const int OFF_W4 = OFF_BIAS + 4 * MLP_H * 4;
 const int STEP_SMEM = OFF_W4 + MLP_H * MLP_OUT * 4;
 const int NGEMM = 6;  // the hidden layers forward, then back
-
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-// barrier that returns the conjunction of the threads' flags
-__device__ __forceinline__ bool bar_and(int id, int n, bool f)
-{
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.and.pred q, %2, %3, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(r)
-        : "r"((uint32_t)f), "r"(id), "r"(n)
-        : "memory");
-    return r != 0;
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(bar)) : "memory");
-}
 
 // One step of a sum shared out over lanes: the lane with bit 4 W set keeps
 // entries W .. 2 W - 1 of the pair's sums, the other 0 .. W - 1 (in s[0..W))
@@ -208,7 +168,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
 #pragma unroll 1
                 for (int c2 = 0; c2 < 2 * NCHUNK; ++c2, ++q) {
                     const int c = c2 % NCHUNK, s = (int)(q % RING);
-                    if (q >= RING) ok = ctl_wait(&empty[s], (q / RING - 1) & 1);
+                    if (q >= RING) ok = tc_poll_wait(&empty[s], (q / RING - 1) & 1);
                     if (!ok) break;
                     tc_load_warp(smem + OFF_RING + s * CHUNK_BYTES, w + (size_t)c * MLP_H * MLP_KC, CHUNK_BYTES,
                                  CHUNK_BYTES, &full[s]);
@@ -225,7 +185,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
             for (int g = 0; g < NGEMM && ok; ++g, ++nready) {
 #pragma unroll 1
                 for (int t = 0; t < 2 && ok; ++t) {
-                    ok = ctl_wait(&ready[t], nready & 1);
+                    ok = tc_poll_wait(&ready[t], nready & 1);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t da = tc_desc(tc_smem(smem + t * TILE_BYTES), 128, (MLP_H / 8) * 128);
@@ -233,7 +193,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
 #pragma unroll 1
                     for (int c = 0; c < NCHUNK; ++c, ++q) {
                         const int s = (int)(q % RING);
-                        ok = ctl_wait(&full[s], (q / RING) & 1);
+                        ok = tc_poll_wait(&full[s], (q / RING) & 1);
                         if (!ok) break;
                         tc_fence_after();
                         const uint64_t db = tc_desc(tc_smem(smem + OFF_RING + s * CHUNK_BYTES), 128, (MLP_KC / 8) * 128);
@@ -263,11 +223,11 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
             tc_fence_proxy_async();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&ready[t]);
+            if (lane == 0) tc_arrive(&ready[t]);
         };
         auto take = [&]() -> bool {
             // the tile's threads agree, so that none waits for one that gave up
-            if (!bar_and(bar_tile, 256, ctl_wait(&done[t], ngemm & 1))) return false;
+            if (!tc_bar_and(bar_tile, 256, tc_poll_wait(&done[t], ngemm & 1))) return false;
             ++ngemm;
             tc_fence_after();
             return true;
@@ -289,7 +249,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
             const int tt = tid & 255;
             *(float4 *)(sX + tt * 4) = load_row4(a.X + (size_t)tile * TILE * MLP_XS + tt * 4, a.aligned);
             const float4 tg = load_row4(a.T + gr * MLP_OUT, a.aligned), wt = load_row4(a.w + gr * MLP_OUT, a.aligned);
-            bar_sync(bar_tile, 256);
+            tc_bar_sync(bar_tile, 256);
             // ---- as exact sums of three bf16 pieces, and a one (the bias): the
             // operand of the input layer's gradient ----
             if (half == 0) {
@@ -428,7 +388,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
                     }
                     sY[row] = make_float4(y01.x, y01.y, y23.x, y23.y);
                 }
-                bar_sync(bar_tile, 256);
+                tc_bar_sync(bar_tile, 256);
             }
             float4 d;
             {
@@ -446,7 +406,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
                     gb4[0] += d.x, gb4[1] += d.y, gb4[2] += d.z, gb4[3] += d.w;
                 }
             }
-            bar_sync(bar_tile, 256);
+            tc_bar_sync(bar_tile, 256);
             // ---- dW4: sums over rows ----
             // 16 columns of a tile half at a time go through shared memory (16-byte
             // units permuted in each pair of rows: no bank conflicts either way);
@@ -462,7 +422,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
                 float4 dd[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) dd[i] = sDY[r0 + i];
-                bar_sync(bar_tile, 256);  // the staging takes the place of y and dY
+                tc_bar_sync(bar_tile, 256);  // the staging takes the place of y and dY
 #pragma unroll 1
                 for (int c = 0; c < 8; ++c) {
                     float v[16];
@@ -470,7 +430,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
                         *(float4 *)(stg + unit(row, u)) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
-                    bar_sync(bar_half, 128);
+                    tc_bar_sync(bar_half, 128);
                     float2 s[8] = {};  // [column][output pair]
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
@@ -491,7 +451,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
 #pragma unroll
                     for (int k = 0; k < 7; ++k) gw4[k] = gw4[k + 1];
                     gw4[7] = g;
-                    bar_sync(bar_half, 128);
+                    tc_bar_sync(bar_half, 128);
                 }
             }
             // ---- dZ4 = (dY W4^T) gelu' ----
@@ -555,7 +515,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
         }
         // ---- this CTA's sums of dW4, db4 and the loss, in a fixed order ----
         if (!ok) atomicExch(a.err, -9);
-        bar_sync(7, 512);
+        tc_bar_sync(7, 512);
         float *red = (float *)smem;  // [tile][row quarter][half * 128 + column][4], then the row sums
 #pragma unroll
         for (int c = 0; c < 8; ++c)
@@ -571,7 +531,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
         if (half == 0 && lane == 0)
 #pragma unroll
             for (int k = 0; k < 5; ++k) rs[(t * 4 + (warp & 3)) * 5 + k] = s5[k];
-        bar_sync(7, 512);
+        tc_bar_sync(7, 512);
         float *po = a.b.part_o + (size_t)blockIdx.x * PB_O;
         for (int i = tid; i < MLP_H * MLP_OUT; i += 512) {
             float s = 0.f;
@@ -671,7 +631,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) mlp_grad_kernel(const GradArg
 #pragma unroll 1
         for (; i < n; ++i) {
             const int st = i % GSTAGES;
-            if (!(ok = ctl_wait(&full[st], (uint32_t)(i / GSTAGES) & 1))) break;
+            if (!(ok = tc_poll_wait(&full[st], (uint32_t)(i / GSTAGES) & 1))) break;
             tc_fence_after();
             const uint32_t a0 = tc_smem(smem + st * (GA_BYTES + GB_BYTES));
             // MN-major, no swizzle: 8-feature groups 128 bytes apart (the
@@ -687,7 +647,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) mlp_grad_kernel(const GradArg
             tc_commit_warp(&empty[st]);
             if (i > 0 && loaded < n) {
                 const int p = i - 1;
-                if (!(ok = ctl_wait(&empty[p % GSTAGES], (uint32_t)(p / GSTAGES) & 1))) break;
+                if (!(ok = tc_poll_wait(&empty[p % GSTAGES], (uint32_t)(p / GSTAGES) & 1))) break;
                 load(loaded++);
             }
         }

@@ -99,3 +99,30 @@ def test_training_step_tiles(n, offset):
     assert abs(loss - lo) <= 1e-3 * lo
     for name, (a, b) in param_slices().items():
         assert relerr(g[a:b], go[a:b]) <= 2e-3, name
+
+
+@pytest.mark.parametrize("nx,ny,footprint,levels", [
+    (501, 533, True, 8),            # odd mode counts (clamped), pairs of modes per thread
+    (512, 560, True, 8),            # even, with the unpaired Nyquist row and column
+    (460, 512, False, [0, 3, 8]),   # a source spectrum and several output levels
+    (20, 6, False, [0, 3, 8]),      # one mode per thread, fewer modes than a block
+    (3, 2, True, 4),                # the smallest grids
+])
+def test_fp64_sweep_items(nx, ny, footprint, levels):
+    """Both FP64 sweeps over every mode of grids with odd and even mode counts,
+    above and below the size where a thread takes two modes: 1e-10 against the
+    oracle (reference rounding), 1e-11 against its invariant imbedding."""
+    from bldfm_gb300 import steady_state_transport_solver
+
+    z, p = O.vertical_profiles(8, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    rng = np.random.default_rng(nx)
+    src = np.zeros((ny, nx)) if footprint else rng.uniform(0.0, 1.0, (ny, nx))
+    kw = dict(srf_flx=src, z=z, profiles=p, domain=(4.0 * nx, 4.0 * ny), levels=levels,
+              modes=(2 * nx, 2 * ny) if footprint else (nx, ny), meas_pt=(3.0, 2.0), footprint=footprint, halo=0.0,
+              precision="double")
+    _, c, f = steady_state_transport_solver(**kw)
+    _, oc, of = O.steady_state_transport_solver(**kw)
+    assert relerr(c, oc) <= 1e-10 and relerr(f, of) <= 1e-10
+    _, c, f = steady_state_transport_solver(**kw, mode="fp64r")
+    _, oc, of = O.steady_state_transport_solver(**kw, sweep="riccati")
+    assert relerr(c, oc) <= 1e-11 and relerr(f, of) <= 1e-11
