@@ -673,12 +673,14 @@ __global__ void __launch_bounds__(128) riccati64_kernel(SolveGeom g, const doubl
 }
 
 // Modes per thread and threads per block of the FP64 sweeps.  The pipe passes
-// one instruction per 16 clocks and SM, whatever its warps, so a launch takes
-// (warps of the fullest SM) x (instructions of a warp): one1 for a warp of
-// single modes, one2 of pairs.  Pairs issue fewer in all but come in coarser
-// units, and reach 95% of the pipe's rate (single modes 99%).  Small blocks
-// spread a small solve evenly (256^2 modes: 772 us in blocks of one warp, 877
-// in blocks of four), larger ones where the level table leaves room for few.
+// one instruction per 16 clocks and SM, but of one warp only one per 64, so a
+// launch takes (warps of the fullest SM, at least 4) x (instructions of a
+// warp): one1 for a warp of single modes, one2 of pairs.  Pairs issue fewer in
+// all but come in coarser units, and reach 95% of the pipe's rate (single modes
+// 99%): 128^2 modes over 47 levels take 106 us as singles, 191 us as pairs,
+// 384^2 modes 885 and 821.  Small blocks spread a small solve evenly (256^2
+// modes: 772 us in blocks of one warp, 877 in blocks of four), larger ones
+// where the level table leaves room for few.
 struct Sweep64Launch {
     bool pairs;
     int threads;
@@ -688,7 +690,7 @@ struct Sweep64Launch {
 static Sweep64Launch sweep64_launch(const SolveGeom &g, size_t smem, int nsm, double one1, double one2)
 {
     const int64_t n2 = sweep_items(g.nlx, g.nly).n;
-    auto units = [&](int64_t n) { return (double)(((n + 31) / 32 + nsm - 1) / nsm); };
+    auto units = [&](int64_t n) { return (double)std::max<int64_t>(((n + 31) / 32 + nsm - 1) / nsm, 4); };
     Sweep64Launch l;
     l.pairs = units(n2) * one2 < 0.95 * units(g.nsolved) * one1;
     const int64_t n = l.pairs ? n2 : g.nsolved;
