@@ -704,6 +704,11 @@ struct BatchBuild {
     std::vector<int4 *> xb;
     size_t off_cases = 0, off_tile_case = 0, off_cta_tiles = 0, off_col_case = 0, off_row_case = 0;
     std::vector<size_t> off_lv32, off_lv64, off_lvd, off_slot, off_dc;
+    // dispersion cases: their indices, the FwdCase table, its launch
+    std::vector<int> disp;
+    size_t off_fwd = 0, fwd_row_smem = 0, fwd_col_smem = 0;
+    int fwd_rows = 0, fwd_cols = 0, fwd_nz = 0;
+    std::vector<int> fwd_rpc, fwd_cpc;
     size_t blob_bytes = 0, blob_at = 0, extra_off = 0;
     std::vector<size_t> d_q0, d_A, d_dcp, d_scratch, d_Xp, d_Xq, d_Cb;
     size_t total = 0;
@@ -878,6 +883,10 @@ int batch_build(const bldfm_case *cs, int n, const bldfm_batch_opts *opts, Devic
         B.off_dc[k] = o;
         o = al(o + (size_t)g.nlvls * 32);
     }
+    for (int k = 0; k < n; ++k)
+        if (!B.hp[k].g.footprint) B.disp.push_back(k);
+    B.off_fwd = o;
+    o = al(o + sizeof(FwdCase) * B.disp.size());
     B.extra_off = o;  // caller's region at the end of the blob
     o = al(o + extra_blob);
     B.blob_bytes = o;
@@ -942,6 +951,25 @@ int batch_build(const bldfm_case *cs, int n, const bldfm_batch_opts *opts, Devic
     }
     if (B.sweep_smem > 200 * 1024) return BLDFM_ERR_UNSUPPORTED;
     if (!dc) return BLDFM_OK;
+    // forward passes of the dispersion cases: lines per block, blocks of the
+    // largest case, shared memory
+    B.fwd_rpc.assign(n, 1);
+    B.fwd_cpc.assign(n, 1);
+    int64_t lr = 0, lc = 0;
+    for (int k : B.disp) {
+        lr += B.hp[k].g.ny;
+        lc += B.hp[k].g.nlx;
+    }
+    for (int k : B.disp) {
+        const HostPlan &hp = B.hp[k];
+        const int r = B.fwd_rpc[k] = fwd_lines_per_cta(hp.plx_fwd.n, 8, (int)std::min<int64_t>(lr, INT_MAX), dc->nsm);
+        const int c = B.fwd_cpc[k] = fwd_lines_per_cta(hp.ply_fwd.n, 8, (int)std::min<int64_t>(lc, INT_MAX), dc->nsm);
+        B.fwd_rows = std::max(B.fwd_rows, (hp.g.ny + r - 1) / r);
+        B.fwd_cols = std::max(B.fwd_cols, (hp.g.nlx + c - 1) / c);
+        B.fwd_row_smem = std::max(B.fwd_row_smem, fwd_smem(hp.plx_fwd.n, 8, r));
+        B.fwd_col_smem = std::max(B.fwd_col_smem, fwd_smem(hp.ply_fwd.n, 8, c));
+        B.fwd_nz = std::max(B.fwd_nz, hp.g.nz);
+    }
     // persistent sweep grid
     int per_sm = (opts && opts->ctas_per_sm > 0) ? opts->ctas_per_sm : batch_sweep_occupancy(B.threads, B.sweep_smem);
     B.G = (int)std::min<int64_t>(std::min<int64_t>((int64_t)dc->nsm * per_sm, BATCH_MAX_CTAS),
@@ -1039,6 +1067,28 @@ void batch_fill_blob(const bldfm_case *cs, int n, BatchBuild &B, char *ws, char 
         for (int64_t i = 0; i < (int64_t)g.nlvls * nblk; ++i) row_case[B.rowbase[k] + B.row0[k] + i] = k;
     };
     HostPool::get().run(n, one_case);
+    FwdCase *fw = (FwdCase *)(blob + B.off_fwd);
+    for (size_t i = 0; i < B.disp.size(); ++i) {
+        const int k = B.disp[i];
+        const HostPlan &hp = B.hp[k];
+        FwdCase &f = fw[i];
+        memset(&f, 0, sizeof(f));
+        f.g = hp.g;
+        f.plx = hp.plx_fwd;
+        f.ply = hp.ply_fwd;
+        f.twx = B.twxf[k]->d32;
+        f.twy = B.twyf[k]->d32;
+        f.src = cs[k].srf_flx_dev;
+        f.A = (float2 *)(ws + B.d_A[k]);
+        f.Q0 = (float2 *)(ws + B.d_q0[k]);
+        f.lv64 = (const double *)(wb + B.off_lv64[k]);
+        f.slot = (const int *)(wb + B.off_slot[k]);
+        f.dc = (double2 *)(wb + B.off_dc[k]);
+        f.dcp = (double *)(ws + B.d_dcp[k]);
+        f.p000 = cs[k].desc.srf_bg_conc;
+        f.rpc = B.fwd_rpc[k];
+        f.cpc = B.fwd_cpc[k];
+    }
     // cost-weighted contiguous partition of the tiles over G persistent CTAs
     std::vector<double> tile_cost;
     tile_cost.reserve((size_t)B.ntiles);
@@ -1075,14 +1125,21 @@ int batch_enqueue(const bldfm_case *cs, int n, BatchBuild &B, char *ws, const vo
             CK(cudaMemsetAsync(ws + B.d_Xp[k], 0, specb, st));
             CK(cudaMemsetAsync(ws + B.d_Xq[k], 0, specb, st));
         }
-        if (!g.footprint) {
-            float2 *q0 = (float2 *)(ws + B.d_q0[k]);
-            CK(launch_forward_fft<float>(g, B.hp[k].plx_fwd, B.hp[k].ply_fwd, B.twxf[k]->d32, B.twyf[k]->d32,
-                                         cs[k].srf_flx_dev, (float2 *)(ws + B.d_A[k]), q0, st));
-            CK(launch_trapezoid32(g, (const double *)(wb + B.off_lv64[k]), (const int *)(wb + B.off_slot[k]), q0,
-                                  cs[k].desc.srf_bg_conc, (double2 *)(wb + B.off_dc[k]), st, cs[k].srf_flx_dev,
-                                  (double *)(ws + B.d_dcp[k])));
+    }
+    // the k = 0 values of the dispersion cases read only the sources and the
+    // level tables: they run on the auxiliary stream beside the forward
+    // transforms and the sweep
+    const bool disp = !B.disp.empty(), side = aux && !tdc;
+    if (disp) {
+        const FwdCase *fw = (const FwdCase *)(wb + B.off_fwd);
+        const int nd = (int)B.disp.size();
+        if (side) {
+            CK(cudaEventRecord(aux->fork, st));
+            CK(cudaStreamWaitEvent(aux->s, aux->fork, 0));
         }
+        CK(launch_dc_batch(fw, nd, B.fwd_nz, side ? aux->s : st));
+        if (side) CK(cudaEventRecord(aux->join, aux->s));
+        CK(launch_forward_batch(fw, nd, B.fwd_rows, B.fwd_row_smem, B.fwd_cols, B.fwd_col_smem, st));
     }
     BatchLaunch bl;
     bl.cases = (const BatchCase *)(wb + B.off_cases);
@@ -1110,10 +1167,11 @@ int batch_enqueue(const bldfm_case *cs, int n, BatchBuild &B, char *ws, const vo
     for (int i = 0; i < B.nxg; ++i) bl.xg[i] = B.xg[i];
     if (tdc) tmark(*tdc, st);  // 1: the sweep
     CK(launch_batch_kernels(bl, st, 0));
+    if (disp && side) CK(cudaStreamWaitEvent(st, aux->join, 0));
     // the accuracy check reads the spectra, as the transform passes do: it
     // runs beside them on the auxiliary stream (after them when the stages
     // are timed, so that each stage's time is its own)
-    const bool fork = B.check && aux && !tdc;
+    const bool fork = B.check && side;
     if (fork) {
         CK(cudaEventRecord(aux->fork, st));
         CK(cudaStreamWaitEvent(aux->s, aux->fork, 0));

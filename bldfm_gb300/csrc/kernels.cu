@@ -276,21 +276,12 @@ __global__ void __launch_bounds__(256) combine64_kernel(SolveGeom g, const uint3
 // dcp (may be NULL): DC_PARTS partial FP64 sums of the source field
 // (dc_partial_kernel); the k = 0 source value is then their sum / (nxe nye)
 // in FP64 instead of the transform's k = 0 output.
-template <typename C>
-__global__ void __launch_bounds__(256) trapezoid_kernel(SolveGeom g, const double *__restrict__ lvtab,
-                                                        const int *__restrict__ slot_of_step,
-                                                        const C *__restrict__ q0spec, double p000,
-                                                        double2 *__restrict__ dc, const double *__restrict__ dcp)
+__device__ __forceinline__ void trapezoid_values(const SolveGeom &g, const double *__restrict__ lvtab,
+                                                 const int *__restrict__ slot_of_step, double2 q0, double p000,
+                                                 double2 *__restrict__ dc, unsigned char *smem_raw)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     double2 *term = (double2 *)smem_raw;
     int *sl = (int *)(term + (g.nz > 1 ? g.nz - 1 : 1));
-    double2 q0 = make_double2((double)q0spec[0].x, (double)q0spec[0].y);
-    if (dcp) {
-        double sum = 0.0;
-        for (int b = 0; b < DC_PARTS; ++b) sum += dcp[b];
-        q0 = make_double2(sum * g.inv_nxe * g.inv_nye, 0.0);
-    }
     const bool single = g.precision == 0;
     const double2 qs = single ? round_c64(q0) : q0;
     for (int s = threadIdx.x; s < g.nlvls; s += blockDim.x) {
@@ -316,6 +307,32 @@ __global__ void __launch_bounds__(256) trapezoid_kernel(SolveGeom g, const doubl
     }
     const int s = sl[g.nz - 1];
     if (s >= 0) dc[2 * s] = single ? round_c64(p00) : p00;
+}
+
+template <typename C>
+__global__ void __launch_bounds__(256) trapezoid_kernel(SolveGeom g, const double *__restrict__ lvtab,
+                                                        const int *__restrict__ slot_of_step,
+                                                        const C *__restrict__ q0spec, double p000,
+                                                        double2 *__restrict__ dc, const double *__restrict__ dcp)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2 q0 = make_double2((double)q0spec[0].x, (double)q0spec[0].y);
+    if (dcp) {
+        double sum = 0.0;
+        for (int b = 0; b < DC_PARTS; ++b) sum += dcp[b];
+        q0 = make_double2(sum * g.inv_nxe * g.inv_nye, 0.0);
+    }
+    trapezoid_values(g, lvtab, slot_of_step, q0, p000, dc, smem_raw);
+}
+
+// the k = 0 values of a batch's dispersion cases, one block per case
+__global__ void __launch_bounds__(256) trapezoid_batch_kernel(const FwdCase *__restrict__ cases)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const FwdCase &c = cases[blockIdx.x];
+    double sum = 0.0;
+    for (int b = 0; b < DC_PARTS; ++b) sum += c.dcp[b];
+    trapezoid_values(c.g, c.lv64, c.slot, make_double2(sum * c.g.inv_nxe * c.g.inv_nye, 0.0), c.p000, c.dc, smem_raw);
 }
 
 // ---------------------------------------------------------------------------
@@ -720,26 +737,28 @@ cudaError_t launch_riccati64(const SolveGeom &g, const double *lvtab, const int 
 // FFT passes
 // ---------------------------------------------------------------------------
 // fwd_rows: lines are source rows y < ny, length nxe, input at offset px.
-// Output A[c][y] (c < nlx truncated columns) scaled by 1/nxe.
+// Output A[c][y] (c < nlx truncated columns) scaled by 1/nxe.  smem: two
+// ping-pong buffers of rows_per_cta lines, then the twiddles.
 template <typename R>
-__global__ void __launch_bounds__(256) fwd_rows_kernel(SolveGeom g, FftPlan pl, const typename cvec<R>::T *__restrict__ tw,
-                                                       const double *__restrict__ src, typename cvec<R>::T *__restrict__ A,
-                                                       int rows_per_cta)
+__device__ __forceinline__ void fwd_row_lines(const SolveGeom &g, const FftPlan &pl,
+                                              const typename cvec<R>::T *__restrict__ tw,
+                                              const double *__restrict__ src, typename cvec<R>::T *__restrict__ A,
+                                              int y0, int rows_per_cta, typename cvec<R>::T *smem)
 {
     typedef typename cvec<R>::T C;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = pl.n;
-    C *bufA = (C *)smem_raw;
+    C *bufA = smem;
     C *bufB = bufA + (size_t)rows_per_cta * n;
-    const int y0 = blockIdx.x * rows_per_cta;
+    C *stw = bufB + (size_t)rows_per_cta * n;
     const int nl = min(rows_per_cta, g.ny - y0);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) stw[i] = tw[i];
     for (int i = threadIdx.x; i < nl * n; i += blockDim.x) {
         const int l = i / n, x = i - l * n;
         const int xs = x - g.px;
         R v = (xs >= 0 && xs < g.nx) ? (R)src[(size_t)(y0 + l) * g.nx + xs] : (R)0;
         bufA[i] = cx_make<C>(v, 0.0);
     }
-    C *res = fft_run<C>(bufA, bufB, pl, nl, tw, -1);
+    C *res = fft_run<C>(bufA, bufB, pl, nl, stw, -1);
     const R sc = (R)g.inv_nxe;
     for (int i = threadIdx.x; i < nl * g.nlx; i += blockDim.x) {
         const int c = i / nl, l = i - c * nl;
@@ -755,23 +774,25 @@ __global__ void __launch_bounds__(256) fwd_rows_kernel(SolveGeom g, FftPlan pl, 
 // fwd_cols: lines are truncated columns c < nlx, length nye, input A[c][y] at
 // offset py.  Output Q0[c][r] (r < nly) scaled by 1/nye.
 template <typename R>
-__global__ void __launch_bounds__(256) fwd_cols_kernel(SolveGeom g, FftPlan pl, const typename cvec<R>::T *__restrict__ tw,
-                                                       const typename cvec<R>::T *__restrict__ A,
-                                                       typename cvec<R>::T *__restrict__ Q0, int cols_per_cta)
+__device__ __forceinline__ void fwd_col_lines(const SolveGeom &g, const FftPlan &pl,
+                                              const typename cvec<R>::T *__restrict__ tw,
+                                              const typename cvec<R>::T *__restrict__ A,
+                                              typename cvec<R>::T *__restrict__ Q0, int c0, int cols_per_cta,
+                                              typename cvec<R>::T *smem)
 {
     typedef typename cvec<R>::T C;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = pl.n;
-    C *bufA = (C *)smem_raw;
+    C *bufA = smem;
     C *bufB = bufA + (size_t)cols_per_cta * n;
-    const int c0 = blockIdx.x * cols_per_cta;
+    C *stw = bufB + (size_t)cols_per_cta * n;
     const int nl = min(cols_per_cta, g.nlx - c0);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) stw[i] = tw[i];
     for (int i = threadIdx.x; i < nl * n; i += blockDim.x) {
         const int l = i / n, y = i - l * n;
         const int ys = y - g.py;
         bufA[i] = (ys >= 0 && ys < g.ny) ? A[(size_t)(c0 + l) * g.ny + ys] : cx_make<C>(0.0, 0.0);
     }
-    C *res = fft_run<C>(bufA, bufB, pl, nl, tw, -1);
+    C *res = fft_run<C>(bufA, bufB, pl, nl, stw, -1);
     const R sc = (R)g.inv_nye;
     for (int i = threadIdx.x; i < nl * g.nly; i += blockDim.x) {
         const int l = i / g.nly, r = i - l * g.nly;
@@ -782,6 +803,54 @@ __global__ void __launch_bounds__(256) fwd_cols_kernel(SolveGeom g, FftPlan pl, 
         v.y *= sc;
         Q0[(size_t)(c0 + l) * g.nly + r] = v;
     }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) fwd_rows_kernel(SolveGeom g, FftPlan pl, const typename cvec<R>::T *__restrict__ tw,
+                                                       const double *__restrict__ src, typename cvec<R>::T *__restrict__ A,
+                                                       int rows_per_cta)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    fwd_row_lines<R>(g, pl, tw, src, A, blockIdx.x * rows_per_cta, rows_per_cta, (typename cvec<R>::T *)smem_raw);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) fwd_cols_kernel(SolveGeom g, FftPlan pl, const typename cvec<R>::T *__restrict__ tw,
+                                                       const typename cvec<R>::T *__restrict__ A,
+                                                       typename cvec<R>::T *__restrict__ Q0, int cols_per_cta)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    fwd_col_lines<R>(g, pl, tw, A, Q0, blockIdx.x * cols_per_cta, cols_per_cta, (typename cvec<R>::T *)smem_raw);
+}
+
+// The forward passes of a batch's dispersion cases, blockIdx.y = case: one
+// launch per pass (per-case launches of some 30 blocks each, one after
+// another, left most of the device idle: 136 us for four 256 x 192 sources,
+// 26 us so).
+__device__ __forceinline__ void load_fwd_case(FwdCase *dst, const FwdCase *src)
+{
+    const int *s = (const int *)src;
+    int *d = (int *)dst;
+    for (int i = threadIdx.x; i < (int)(sizeof(FwdCase) / 4); i += blockDim.x) d[i] = s[i];
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) fwd_rows_batch_kernel(const FwdCase *__restrict__ cases)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(16) FwdCase fc;
+    if ((int)blockIdx.x * cases[blockIdx.y].rpc >= cases[blockIdx.y].g.ny) return;
+    load_fwd_case(&fc, cases + blockIdx.y);
+    fwd_row_lines<float>(fc.g, fc.plx, fc.twx, fc.src, fc.A, blockIdx.x * fc.rpc, fc.rpc, (float2 *)smem_raw);
+}
+
+__global__ void __launch_bounds__(256) fwd_cols_batch_kernel(const FwdCase *__restrict__ cases)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(16) FwdCase fc;
+    if ((int)blockIdx.x * cases[blockIdx.y].cpc >= cases[blockIdx.y].g.nlx) return;
+    load_fwd_case(&fc, cases + blockIdx.y);
+    fwd_col_lines<float>(fc.g, fc.ply, fc.twy, fc.A, fc.Q0, blockIdx.x * fc.cpc, fc.cpc, (float2 *)smem_raw);
 }
 
 // out_cols: cols_per_cta band columns per CTA (blockIdx.x), one level (blockIdx.y).
@@ -901,8 +970,7 @@ cudaError_t launch_trapezoid64(const SolveGeom &g, const double *lvtab, const in
 
 // FP64 partial sums of the source field: CTA b of DC_PARTS sums its slice in a
 // fixed order (deterministic), thread sums then a shared-memory tree
-__global__ void __launch_bounds__(256) dc_partial_kernel(const double *__restrict__ src, int64_t n,
-                                                         double *__restrict__ dcp)
+__device__ __forceinline__ void dc_partial_sum(const double *__restrict__ src, int64_t n, double *__restrict__ dcp)
 {
     __shared__ double red[256];
     const int64_t chunk = (n + DC_PARTS - 1) / DC_PARTS;
@@ -916,6 +984,18 @@ __global__ void __launch_bounds__(256) dc_partial_kernel(const double *__restric
         __syncthreads();
     }
     if (threadIdx.x == 0) dcp[blockIdx.x] = red[0];
+}
+
+__global__ void __launch_bounds__(256) dc_partial_kernel(const double *__restrict__ src, int64_t n,
+                                                         double *__restrict__ dcp)
+{
+    dc_partial_sum(src, n, dcp);
+}
+
+__global__ void __launch_bounds__(256) dc_partial_batch_kernel(const FwdCase *__restrict__ cases)
+{
+    const FwdCase &c = cases[blockIdx.y];
+    dc_partial_sum(c.src, (int64_t)c.g.nx * c.g.ny, c.dcp);
 }
 
 cudaError_t launch_trapezoid32(const SolveGeom &g, const double *lvtab, const int *slot, const float2 *q0spec,
@@ -979,13 +1059,26 @@ cudaError_t launch_riccati32(const SolveGeom &g, const float *lv32, const int *s
     return LAUNCH_CHECK();
 }
 
-static int lines_per_cta(int n, size_t elem, size_t budget)
+static int device_sms()
 {
-    int l = (int)(budget / (2 * (size_t)n * elem));
-    if (l < 1) l = 1;
-    if (l > 8) l = 8;
+    int dev = 0, nsm = 152;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
+}
+
+// Lines of a forward pass per block: as many as fit about 96 KB, at most 8,
+// but at least two blocks per SM over the launch (a single source has few
+// lines: the two passes of 190 x 150 in FP64 took 136 us at up to eight lines a
+// block, 52 us so).
+int fwd_lines_per_cta(int n, size_t elem, int lines, int nsm)
+{
+    int l = (int)((96 * 1024) / (2 * (size_t)n * elem));
+    l = std::min(std::max(l, 1), 8);
+    while (l > 1 && (lines + l - 1) / l < 2 * nsm) --l;
     return l;
 }
+
+size_t fwd_smem(int n, size_t elem, int lines) { return (2 * (size_t)lines + 1) * n * elem; }
 
 template <typename R>
 static void set_fft_smem_attr()
@@ -996,6 +1089,10 @@ static void set_fft_smem_attr()
     cudaFuncSetAttribute(fwd_cols_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(out_cols_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(out_rows_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (sizeof(R) == 4) {
+        cudaFuncSetAttribute(fwd_rows_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(fwd_cols_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    }
 }
 
 template <typename R>
@@ -1006,13 +1103,11 @@ cudaError_t launch_forward_fft(const SolveGeom &g, const FftPlan &plx, const Fft
     typedef typename cvec<R>::T C;
     set_fft_smem_attr<R>();
     if (g.ny <= 0 || g.nlx <= 0) return cudaSuccess;
-    const size_t budget = 96 * 1024;
-    int rpc = lines_per_cta(plx.n, sizeof(C), budget);
-    fwd_rows_kernel<R><<<(g.ny + rpc - 1) / rpc, 256, 2 * (size_t)rpc * plx.n * sizeof(C), st>>>(g, plx, twx, src, A,
-                                                                                                  rpc);
-    int cpc = lines_per_cta(ply.n, sizeof(C), budget);
-    fwd_cols_kernel<R><<<(g.nlx + cpc - 1) / cpc, 256, 2 * (size_t)cpc * ply.n * sizeof(C), st>>>(g, ply, twy, A, Q0,
-                                                                                                   cpc);
+    const int nsm = device_sms();
+    const int rpc = fwd_lines_per_cta(plx.n, sizeof(C), g.ny, nsm);
+    fwd_rows_kernel<R><<<(g.ny + rpc - 1) / rpc, 256, fwd_smem(plx.n, sizeof(C), rpc), st>>>(g, plx, twx, src, A, rpc);
+    const int cpc = fwd_lines_per_cta(ply.n, sizeof(C), g.nlx, nsm);
+    fwd_cols_kernel<R><<<(g.nlx + cpc - 1) / cpc, 256, fwd_smem(ply.n, sizeof(C), cpc), st>>>(g, ply, twy, A, Q0, cpc);
     return LAUNCH_CHECK();
 }
 
@@ -1027,8 +1122,7 @@ cudaError_t launch_output_fft(const SolveGeom &g, const FftPlan &plx, const FftP
     if (g.nbx <= 0 || g.out_ny <= 0 || g.out_nx <= 0 || g.nlvls <= 0) return cudaSuccess;
     // lines per CTA: as many as shared memory allows, but at least two CTAs
     // per SM over the launch (a single footprint has few lines)
-    int dev = 0, nsm = 152;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int nsm = device_sms();
     int cpc = out_cols_per_cta(ply.n, sizeof(C));
     while (cpc > 1 && (int64_t)((g.nbx + cpc - 1) / cpc) * g.nlvls < 2 * (int64_t)nsm) cpc >>= 1;
     dim3 gc((g.nbx + cpc - 1) / cpc, g.nlvls);
@@ -1042,6 +1136,24 @@ cudaError_t launch_output_fft(const SolveGeom &g, const FftPlan &plx, const FftP
     dim3 gr((g.out_ny + rpc - 1) / rpc, g.nlvls);
     out_rows_kernel<R><<<gr, 256, (2 * (size_t)rpc + 1) * plx.n * sizeof(C), st>>>(g, plx, twx, xband, Cbuf, conc,
                                                                                    flx, rpc, err);
+    return LAUNCH_CHECK();
+}
+
+cudaError_t launch_forward_batch(const FwdCase *cases, int n, int rows, size_t row_smem, int cols, size_t col_smem,
+                                 cudaStream_t st)
+{
+    set_fft_smem_attr<float>();
+    fwd_rows_batch_kernel<<<dim3(rows, n), 256, row_smem, st>>>(cases);
+    fwd_cols_batch_kernel<<<dim3(cols, n), 256, col_smem, st>>>(cases);
+    return LAUNCH_CHECK();
+}
+
+cudaError_t launch_dc_batch(const FwdCase *cases, int n, int max_nz, cudaStream_t st)
+{
+    set_fft_smem_attr<float>();
+    dc_partial_batch_kernel<<<dim3(DC_PARTS, n), 256, 0, st>>>(cases);
+    const size_t smem = (size_t)(max_nz > 1 ? max_nz - 1 : 1) * sizeof(double2) + (size_t)max_nz * sizeof(int);
+    trapezoid_batch_kernel<<<n, 256, smem, st>>>(cases);
     return LAUNCH_CHECK();
 }
 

@@ -25,6 +25,29 @@ cudaError_t launch_trapezoid64(const SolveGeom &g, const double *lvtab, const in
 cudaError_t launch_trapezoid32(const SolveGeom &g, const double *lvtab, const int *slot, const float2 *q0spec,
                                double p000, double2 *dc, cudaStream_t st, const double *src = nullptr,
                                double *dcp = nullptr);
+// One dispersion case of a batch: what its forward transform and k = 0 values read
+struct __align__(16) FwdCase {
+    SolveGeom g;
+    FftPlan plx, ply;  // forward transform plans
+    const float2 *twx, *twy;
+    const double *src;
+    float2 *A, *Q0;
+    const double *lv64;
+    const int *slot;
+    double2 *dc;
+    double *dcp;
+    double p000;
+    int32_t rpc, cpc;  // rows, columns per block
+};
+// lines of a forward pass per block for `lines` lines of length n in a launch
+// (elem bytes a complex value), and its shared memory
+int fwd_lines_per_cta(int n, size_t elem, int lines, int nsm);
+size_t fwd_smem(int n, size_t elem, int lines);
+// the forward transforms of n cases (at most rows, cols blocks a case), and
+// their k = 0 values (the source's FP64 sum, then the trapezoid rule)
+cudaError_t launch_forward_batch(const FwdCase *cases, int n, int rows, size_t row_smem, int cols, size_t col_smem,
+                                 cudaStream_t st);
+cudaError_t launch_dc_batch(const FwdCase *cases, int n, int max_nz, cudaStream_t st);
 cudaError_t launch_analytic64(const SolveGeom &g, const uint32_t *modes, const double2 *eig, const double2 *q0spec,
                               double p000, double kzinv, double hlev, double2 *Xp, double2 *Xq, double2 *dc,
                               cudaStream_t st);

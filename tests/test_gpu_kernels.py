@@ -126,3 +126,27 @@ def test_fp64_sweep_items(nx, ny, footprint, levels):
     _, c, f = steady_state_transport_solver(**kw, mode="fp64r")
     _, oc, of = O.steady_state_transport_solver(**kw, sweep="riccati")
     assert relerr(c, oc) <= 1e-11 and relerr(f, of) <= 1e-11
+
+
+@pytest.mark.parametrize("sizes", [
+    [(4, 2)],                              # one line per block, fewer lines than blocks
+    [(64, 48), (4, 2), (150, 302)],        # several cases: the grid is the largest case's
+    [(512, 640), (20, 6)],                 # more lines than two blocks an SM: several per block
+])
+def test_batch_forward_passes(sizes):
+    """Dispersion cases of one batch share the launches of the forward transform
+    and of the k = 0 values: every case, beside a footprint, against the oracle
+    at the bar of the FP32 path, 1e-4."""
+    from bldfm_gb300.batch import solve_batch
+
+    z, p = O.vertical_profiles(8, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    cases = []
+    for i, (nx, ny) in enumerate(sizes + [(32, 24)]):
+        fp = i == len(sizes)
+        src = np.zeros((ny, nx)) if fp else np.random.default_rng(nx).uniform(0.0, 1.0, (ny, nx))
+        cases.append(dict(srf_flx=src, z=z, profiles=p, domain=(4.0 * nx, 4.0 * ny), levels=[2, 8],
+                          modes=(nx, ny), meas_pt=(3.0, 2.0), footprint=fp, halo=8.0, precision="double"))
+    for kw, (_, c, f) in zip(cases, solve_batch(cases)):
+        _, oc, of = O.steady_state_transport_solver(**kw)
+        assert relerr(c.cpu().numpy() if hasattr(c, "cpu") else c, oc) <= 1e-4
+        assert relerr(f.cpu().numpy() if hasattr(f, "cpu") else f, of) <= 1e-4
