@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(256) out_cols_persist_kernel(const BatchCase *
         }
         const int n = sc.ply.n;
         col_line_from_staged(sc.g, bx, sp, sp + sc.g.nly, sc.Xp, sc.Xq, sc.dc, n, lvl, bufA);
-        float2 *res = fft_run<float2>(bufA, bufB, sc.ply, 1, stw, sc.g.out_sign);
+        float2 *res = fft_run<float2>(bufA, bufB, sc.ply, 1, stw, sc.g.out_sign, sc.g.py, sc.g.out_ny);
         float2 *o = sc.Cb + (size_t)lvl * sc.g.out_ny * sc.g.nbx + b;
         for (int y = threadIdx.x; y < sc.g.out_ny; y += blockDim.x) o[(size_t)y * sc.g.nbx] = res[sc.g.py + y];
         __syncthreads();
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(256) out_rows_persist_kernel(const BatchCase *
         }
         for (int bcol = threadIdx.x + PF * (int)blockDim.x; bcol < nb; bcol += blockDim.x)
             bufA[sc.xband[bcol].x] = row[bcol];
-        float2 *res = fft_run<float2>(bufA, bufB, sc.plx, 1, stw, sc.g.out_sign);
+        float2 *res = fft_run<float2>(bufA, bufB, sc.plx, 1, stw, sc.g.out_sign, sc.g.px, sc.g.out_nx);
         const int lvl = local / sc.g.out_ny;
         const int y = local - lvl * sc.g.out_ny;
         const size_t o = ((size_t)lvl * sc.g.out_ny + y) * sc.g.out_nx;

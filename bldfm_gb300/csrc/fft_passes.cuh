@@ -71,7 +71,7 @@ __device__ __forceinline__ void out_col_lines(const SolveGeom &g, const FftPlan 
             line[pos] = cx_make<C>(re, im);
         }
     }
-    C *res = fft_run<C>(bufA, bufB, pl, nc, stw, g.out_sign);
+    C *res = fft_run<C>(bufA, bufB, pl, nc, stw, g.out_sign, g.py, g.out_ny);
     const int lc = 31 - __clz(ncols);  // log2 ncols
     C *o = Cout + (size_t)lvl * g.out_ny * g.nbx + b0;
     for (int i = threadIdx.x; i < (g.out_ny << lc); i += blockDim.x) {
@@ -237,7 +237,7 @@ __device__ __forceinline__ bool out_col_lines_staged(const SolveGeom &g, const F
         const float2 *sp = bufB + (size_t)c * n;
         col_line_from_staged(g, xband[b0 + c], sp, sp + nly, Xp, Xq, dc, n, lvl, bufA + (size_t)c * n);
     }
-    float2 *res = fft_run<float2>(bufA, bufB, pl, nc, stw, g.out_sign);
+    float2 *res = fft_run<float2>(bufA, bufB, pl, nc, stw, g.out_sign, g.py, g.out_ny);
     const int lc = 31 - __clz(ncols);  // log2 ncols
     float2 *o = Cout + (size_t)lvl * g.out_ny * g.nbx + b0;
     for (int i = threadIdx.x; i < (g.out_ny << lc); i += blockDim.x) {
@@ -293,7 +293,7 @@ __device__ __forceinline__ void out_row_lines(const SolveGeom &g, const FftPlan 
         const int l = i / nb, b = i - l * nb;
         bufA[(size_t)l * n + xband[b].x] = rows[i];
     }
-    C *res = fft_run<C>(bufA, bufB, pl, nl, stw, g.out_sign);
+    C *res = fft_run<C>(bufA, bufB, pl, nl, stw, g.out_sign, g.px, g.out_nx);
     bool bad = false;
     for (int i = threadIdx.x; i < nl * g.out_nx; i += blockDim.x) {
         const int l = i / g.out_nx, x = i - l * g.out_nx;

@@ -758,7 +758,8 @@ __device__ __forceinline__ void fwd_row_lines(const SolveGeom &g, const FftPlan 
         R v = (xs >= 0 && xs < g.nx) ? (R)src[(size_t)(y0 + l) * g.nx + xs] : (R)0;
         bufA[i] = cx_make<C>(v, 0.0);
     }
-    C *res = fft_run<C>(bufA, bufB, pl, nl, stw, -1);
+    const int fx = freq_min(g.nlx);
+    C *res = fft_run<C>(bufA, bufB, pl, nl, stw, -1, fx < 0 ? fx + n : fx, g.nlx);
     const R sc = (R)g.inv_nxe;
     for (int i = threadIdx.x; i < nl * g.nlx; i += blockDim.x) {
         const int c = i / nl, l = i - c * nl;
@@ -792,7 +793,8 @@ __device__ __forceinline__ void fwd_col_lines(const SolveGeom &g, const FftPlan 
         const int ys = y - g.py;
         bufA[i] = (ys >= 0 && ys < g.ny) ? A[(size_t)(c0 + l) * g.ny + ys] : cx_make<C>(0.0, 0.0);
     }
-    C *res = fft_run<C>(bufA, bufB, pl, nl, stw, -1);
+    const int fy = freq_min(g.nly);
+    C *res = fft_run<C>(bufA, bufB, pl, nl, stw, -1, fy < 0 ? fy + n : fy, g.nly);
     const R sc = (R)g.inv_nye;
     for (int i = threadIdx.x; i < nl * g.nly; i += blockDim.x) {
         const int l = i / g.nly, r = i - l * g.nly;
