@@ -23,6 +23,7 @@ rounding is added (``error_estimate``).
 """
 
 import ctypes
+import struct
 
 import numpy as np
 import torch
@@ -82,6 +83,49 @@ def _host_inputs(kw):
         levels, lv = _normalise_levels(levels, nz)
         lvp = lv.ctypes.data
     return zp, nz, levels, lv, lvp
+
+
+def _batch_inputs(cases):
+    """:func:`_host_inputs` of every case of a batch and the address of its
+    ``zp``, all inputs in one array where every case has vectors of its own
+    length (one conversion instead of one per case)."""
+
+    def one_by_one():
+        return [h + (h[0].ctypes.data,) for h in map(_host_inputs, cases)]
+
+    flat, nzs = [], []
+    try:
+        for kw in cases:
+            z, p = kw["z"], kw["profiles"]
+            nz = len(z)
+            u, v, kx, ky, kz = p
+            if not len(u) == len(v) == len(kx) == len(ky) == len(kz) == nz:
+                break
+            flat += (z, u, v, kx, ky, kz)
+            nzs.append(nz)
+        if len(nzs) != len(cases) or not nzs:
+            return one_by_one()
+        zps = np.concatenate(flat, dtype=np.float64)
+        if zps.shape != (6 * sum(nzs),):
+            return one_by_one()
+    except (ValueError, TypeError):
+        return one_by_one()
+    out, off, addr = [], 0, zps.ctypes.data
+    for kw, nz in zip(cases, nzs):
+        levels = kw["levels"]
+        if isinstance(levels, (int, np.integer)) and -nz <= int(levels) < nz:
+            lv, lvp, levels = _int_level(levels)
+        else:
+            levels, lv = _normalise_levels(levels, nz)
+            lvp = lv.ctypes.data
+        out.append((zps[off : off + 6 * nz], nz, levels, lv, lvp, addr + 8 * off))
+        off += 6 * nz
+    return out
+
+
+# one C case (Case): descriptor, source, z, profiles, levels, nlvls, padding, conc, flx
+_CASE = struct.Struct("=%ds4Qii2Q" % ctypes.sizeof(_lib.Desc))
+assert _CASE.size == ctypes.sizeof(_lib.Case)
 
 
 # rounding of the FP32 output transform, per unit of the field it transforms:
@@ -152,6 +196,9 @@ class BatchSolver:
         self.opts = _lib.BatchOpts(threads=int(threads), ctas_per_sm=int(ctas_per_sm), use_graph=int(use_graph),
                                    xform_lines=int(xform_lines), skip_check=int(not check))
         self._ws = None
+        self._parts = [0]  # cases per part of the last batch (one part but for solve_batch's large ones)
+        self._more_ws = []  # workspaces of the parts after the first
+        self._copy_stream = None
         self._out_buf = None  # one device buffer holding every case's conc and flx
         self._srf = {}
         self._keep = None
@@ -162,8 +209,16 @@ class BatchSolver:
         if t is None or tuple(t.shape) != a.shape:
             t = torch.empty(a.shape, dtype=torch.float64, device=self.device)
             self._srf[k] = t
-        with torch.cuda.stream(self.stream):
-            t.copy_(torch.from_numpy(a).pin_memory(), non_blocking=True)
+        # one core fills the library's staging ring at 28 GB/s (384 KB: 24 us
+        # against 50 through a pinned tensor); from about 1 MB on torch's
+        # parallel copy into one is the faster
+        if a.nbytes <= 1 << 20:
+            with torch.cuda.device(self.device):
+                _lib.check(_lib.load().bldfm_upload_async(t.data_ptr(), a.ctypes.data, a.nbytes,
+                                                          self.stream.cuda_stream), "solve_batch")
+        else:
+            with torch.cuda.stream(self.stream):
+                t.copy_(torch.from_numpy(a).pin_memory(), non_blocking=True)
         return t
 
     def prepare(self, cases, views=True):
@@ -172,53 +227,58 @@ class BatchSolver:
         views=False skips the torch views of the outputs (outputs is then the
         list of (nlvls, out_ny, out_nx) shapes; the results sit back to back,
         conc then flx per case, at the start of the solver's output buffer)."""
-        n = len(cases)
-        arr = (_lib.Case * n)()
-        outs, keep = [], []
+        metas = self._metas(cases)
+        total = 2 * sum(m[0][2] for m in metas)
+        self._reserve(total)
+        self.out_elems = total
+        return self._fill(cases, metas, views)
+
+    def _metas(self, cases):
+        """Descriptor, output shape and host inputs of each case."""
         metas = []
-        for kw in cases:
-            zp, nz, levels, lv, lvp = _host_inputs(kw)
+        for kw, (zp, nz, levels, lv, lvp, zptr) in zip(cases, _batch_inputs(cases)):
             get = kw.get
             bg = get("srf_bg_conc", 0.0)
             if type(bg) is not float:
                 bg = float(np.real(bg))
-            key = (np.shape(kw["srf_flx"]), nz, tuple(kw["domain"]), tuple(get("modes", (512, 512))),
+            srf = kw["srf_flx"]
+            srf_shape = srf.shape if type(srf) is np.ndarray else np.shape(srf)
+            key = (srf_shape, nz, tuple(kw["domain"]), tuple(get("modes", (512, 512))),
                    tuple(get("meas_pt", (0.0, 0.0))), bg, bool(get("footprint", False)), get("halo"),
                    get("precision", "single"), lv.size)
             hit = _DESC_CACHE.get(key)
             if hit is None:
                 d = make_desc(
-                    np.shape(kw["srf_flx"]), nz, kw["domain"], get("modes", (512, 512)), get("meas_pt", (0.0, 0.0)),
+                    srf_shape, nz, kw["domain"], get("modes", (512, 512)), get("meas_pt", (0.0, 0.0)),
                     get("srf_bg_conc", 0.0), bool(get("footprint", False)), False, get("halo"),
                     get("precision", "single"), "fp32",
                 )
                 info = plan(d, lv.size)
                 shape = (lv.size, info.out_ny, info.out_nx)
-                hit = (d, shape, _count(shape), bool(d.footprint))
+                hit = (bytes(d), shape, _count(shape), bool(d.footprint))
                 if len(_DESC_CACHE) > 256:
                     _DESC_CACHE.clear()
                 _DESC_CACHE[key] = hit
-            metas.append((hit, zp, nz, levels, lv, lvp))
-        total = 2 * sum(m[0][2] for m in metas)
+            metas.append((hit, zp, nz, levels, lv, lvp, zptr))
+        return metas
+
+    def _reserve(self, total):
         if self._out_buf is None or self._out_buf.numel() < total:
             if self._out_buf is not None:  # an earlier batch on the stream may still use it
                 self.stream.synchronize()
             self._out_buf = torch.empty(total, dtype=torch.float64, device=self.device)
-        self.out_elems = total
+
+    def _fill(self, cases, metas, views, off=0, k0=0):
+        """The C descriptors of cases whose outputs start at element off of the
+        output buffer; k0: place of the first one in its batch."""
+        n = len(cases)
+        arr = (_lib.Case * n)()
+        outs, keep = [], []
         base = self._out_buf.data_ptr()
-        off = 0
-        for k, ((d, shape, sz, footprint), zp, nz, levels, lv, lvp) in enumerate(metas):
-            c = arr[k]
-            c.desc = d
-            if not footprint:
-                c.srf_flx_dev = self._srf_dev(k, cases[k]["srf_flx"]).data_ptr()
-            zptr = zp.ctypes.data
-            c.z_host = zptr
-            c.prof_host = zptr + 8 * nz
-            c.levels_host = lvp
-            c.nlvls = lv.size
-            c.conc_dev = base + 8 * off
-            c.flx_dev = base + 8 * (off + sz)
+        for k, ((d, shape, sz, footprint), zp, nz, levels, lv, lvp, zptr) in enumerate(metas):
+            srf = 0 if footprint else self._srf_dev(k0 + k, cases[k]["srf_flx"]).data_ptr()
+            _CASE.pack_into(arr, k * _CASE.size, d, srf, zptr, zptr + 8 * nz, lvp, lv.size, 0, base + 8 * off,
+                            base + 8 * (off + sz))
             if views:
                 ob = self._out_buf
                 outs.append((ob[off : off + sz].view(shape), ob[off + sz : off + 2 * sz].view(shape)))
@@ -236,21 +296,26 @@ class BatchSolver:
         """Enqueue a batch whose C descriptors were built by :meth:`prepare`
         (reusable across calls: the library reads the host arrays at every
         call, so refreshing their contents in place needs no new descriptors)."""
+        self._ws = self._run(prepared, self._ws)
+        self._parts = [len(prepared[0])]
+        self._keep = prepared[2]
+        return prepared[1]
+
+    def _run(self, prepared, ws):
+        """Enqueue a prepared batch on the workspace ws; returns the workspace
+        it ran on (a larger one if ws was too small)."""
         lib = _lib.load()
-        arr, outs, keep = prepared[:3]
+        arr = prepared[0]
         n = len(arr)
 
         def run():
-            return lib.bldfm_solve_batch(
-                arr, n, self.opts, ctypes.c_void_p(self._ws.data_ptr()), ctypes.c_size_t(self._ws.numel()),
-                ctypes.c_void_p(self.stream.cuda_stream),
-            )
+            return lib.bldfm_solve_batch(arr, n, self.opts, ws.data_ptr(), ws.numel(), self.stream.cuda_stream)
 
         # with a workspace in place, solve first: the library checks the size
         # before it touches the stream, so a batch that needs more returns
         # ERR_WORKSPACE with nothing enqueued and is planned and retried
         st = _lib.ERR_WORKSPACE
-        if self._ws is not None and (len(prepared) <= 3 or self._ws.numel() >= prepared[3]):
+        if ws is not None and (len(prepared) <= 3 or ws.numel() >= prepared[3]):
             st = run()
         if st == _lib.ERR_WORKSPACE:
             if len(prepared) > 3:
@@ -259,14 +324,17 @@ class BatchSolver:
                 nb = ctypes.c_int64(0)
                 _lib.check(lib.bldfm_batch_plan(arr, n, self.opts, ctypes.byref(nb)), "solve_batch")
                 need = int(nb.value)
-            if self._ws is None or self._ws.numel() < need:
-                if self._ws is not None:  # an earlier batch on the stream may still use it
+            if ws is None or ws.numel() < need:
+                if ws is not None:  # an earlier batch on the stream may still use it
                     self.stream.synchronize()
-                self._ws = torch.empty(int(need), dtype=torch.uint8, device=self.device)
+                ws = torch.empty(int(need), dtype=torch.uint8, device=self.device)
             st = run()
         _lib.check(st, "solve_batch")
-        self._keep = keep
-        return outs
+        return ws
+
+    def _workspaces(self):
+        """(workspace, cases) of each part of the last batch."""
+        return list(zip([self._ws] + self._more_ws, self._parts))
 
     def prepare_cached(self, cases):
         """:meth:`prepare` plus the workspace size, for repeated solves."""
@@ -281,11 +349,12 @@ class BatchSolver:
         read through this solver's stream only (no device-wide sync)."""
         if self._ws is None:
             return 0
-        st = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        st = torch.empty(len(self._parts), dtype=torch.int32, pin_memory=True)
         with torch.cuda.stream(self.stream):
-            st.copy_(self._ws[:4].view(torch.int32), non_blocking=True)
+            for i, (ws, _) in enumerate(self._workspaces()):
+                st[i : i + 1].copy_(ws[:4].view(torch.int32), non_blocking=True)
         self.stream.synchronize()
-        return int(st[0])
+        return next((int(v) for v in st if v), 0)
 
     def error_estimates(self, n):
         """Estimated relative L2 error of each of the last batch's n cases
@@ -295,13 +364,24 @@ class BatchSolver:
             return np.zeros(0)
         h = torch.empty(16 * n, dtype=torch.uint8, pin_memory=True)
         with torch.cuda.stream(self.stream):
-            h.copy_(self._ws[64 : 64 + 16 * n], non_blocking=True)
+            if len(self._parts) == 1:
+                h.copy_(self._ws[64 : 64 + 16 * n], non_blocking=True)
+            else:
+                k = 0
+                for ws, m in self._workspaces():
+                    m = max(0, min(m, n - k))
+                    h[16 * k : 16 * (k + m)].copy_(ws[64 : 64 + 16 * m], non_blocking=True)
+                    k += m
         self.stream.synchronize()
         return error_estimates(h.view(torch.float32).numpy())
 
 
 _DESC_CACHE = {}  # descriptor and output shape per case geometry
 _grid = output_grid
+
+
+def _memcpy(dst, src, nbytes, stream):
+    _lib.check(_lib.load().bldfm_memcpy_async(dst, src, nbytes, stream.cuda_stream), "solve_batch")
 
 
 def _enqueue_batch(solver, cases):
@@ -312,16 +392,91 @@ def _enqueue_batch(solver, cases):
     nout = 8 * solver.out_elems
     nhead = 64 + 16 * len(cases)
     block = torch.empty(nout + nhead, dtype=torch.uint8, pin_memory=True)
-    host = block[:nout].view(torch.float64)
-    head = block[nout:]
-    lib = _lib.load()
-    s = ctypes.c_void_p(solver.stream.cuda_stream)
     base = block.data_ptr()
-    _lib.check(lib.bldfm_memcpy_async(ctypes.c_void_p(base), ctypes.c_void_p(solver._out_buf.data_ptr()), nout, s),
-               "solve_batch")
-    _lib.check(lib.bldfm_memcpy_async(ctypes.c_void_p(base + nout), ctypes.c_void_p(solver._ws.data_ptr()), nhead,
-                                      s), "solve_batch")
-    return (solver, cases, shapes, solver._keep, host, head)
+    _memcpy(base, solver._out_buf.data_ptr(), nout, solver.stream)
+    _memcpy(base + nout, solver._ws.data_ptr(), nhead, solver.stream)
+    return (solver, cases, shapes, solver._keep, block[:nout].view(torch.float64), block[nout:])
+
+
+PART_BYTES = 12 << 20  # least output bytes of a part of a batch
+MAX_PARTS = 4
+
+
+def _output_bound(kw):
+    """Output elements (conc and flux) of a case, from above: the window is
+    never larger than the source grid."""
+    lv = kw.get("levels", 0)
+    ny, nx = np.shape(kw["srf_flx"])[-2:]
+    return 2 * int(ny) * int(nx) * max(1, int(np.size(lv)))
+
+
+def _split_batch(sizes):
+    """Part boundaries of a batch whose cases have these output bounds (in
+    elements): up to four parts of about equal size and at least 12 MB."""
+    total = sum(sizes)
+    nparts = min(MAX_PARTS, 8 * total // PART_BYTES, len(sizes))
+    cuts, acc = [0], 0
+    for k, v in enumerate(sizes):
+        if len(cuts) < nparts and k > cuts[-1] and acc + v / 2 >= total * len(cuts) / nparts:
+            cuts.append(k)
+        acc += v
+    return cuts + [len(sizes)]
+
+
+def _enqueue_parts(solver, cases):
+    """:func:`_enqueue_batch` for one large batch that the caller waits for: the
+    batch runs as up to four on the solver's stream, each with a workspace of
+    its own, and each part's outputs go back on a second stream while the next
+    part is prepared and computed.  Sixteen towers of 256^2 to 1024^2 (98 MB of
+    results): as one batch 530 us of copying followed the last kernel, as four
+    parts 140 (2121 -> 1927 us)."""
+    try:
+        sizes = [_output_bound(kw) for kw in cases]
+        cuts = _split_batch(sizes)
+    except (TypeError, ValueError, KeyError, IndexError, AttributeError):
+        cuts = [0, len(cases)]  # a malformed case: refused where it is prepared
+    nparts = len(cuts) - 1
+    if nparts < 2:
+        return _enqueue_batch(solver, cases)
+    n = len(cases)
+    solver._reserve(sum(sizes))
+    nout = 8 * sum(sizes)
+    nhead = 64 + 16 * n  # as one batch's; then 64 bytes with the status word of each further part
+    block = torch.empty(nout + nhead + 64 * (nparts - 1), dtype=torch.uint8, pin_memory=True)
+    base, dev = block.data_ptr(), solver._out_buf.data_ptr()
+    if solver._copy_stream is None:
+        solver._copy_stream = torch.cuda.Stream(device=solver.device)
+    cs = solver._copy_stream
+    solver._more_ws += [None] * (nparts - 1 - len(solver._more_ws))
+    shapes, keep, off = [], [], 0
+    try:
+        for i in range(nparts):
+            lo, hi = cuts[i], cuts[i + 1]
+            part = cases[lo:hi]
+            metas = solver._metas(part)
+            prepared = solver._fill(part, metas, False, off, lo)
+            if i == 0:
+                ws = solver._ws = solver._run(prepared, solver._ws)
+            else:
+                ws = solver._more_ws[i - 1] = solver._run(prepared, solver._more_ws[i - 1])
+            cs.wait_stream(solver.stream)
+            cnt = 2 * sum(m[0][2] for m in metas)
+            _memcpy(base + 8 * off, dev + 8 * off, 8 * cnt, cs)
+            _memcpy(base + (nout if i == 0 else nout + nhead + 64 * (i - 1)), ws.data_ptr(), 64, cs)
+            _memcpy(base + nout + 64 + 16 * lo, ws.data_ptr() + 64, 16 * (hi - lo), cs)
+            off += cnt
+            shapes += prepared[1]
+            keep += prepared[2]
+    finally:
+        # the solver's stream goes on only after the copies, and so does a
+        # caller that gets an exception: the pinned block is theirs until then
+        solver.stream.wait_stream(cs)
+        if len(keep) < n:
+            solver.stream.synchronize()
+    solver.out_elems = off
+    solver._parts = [b - a for a, b in zip(cuts, cuts[1:])]
+    solver._keep = keep
+    return (solver, cases, shapes, keep, block[: 8 * off].view(torch.float64), block[nout:])
 
 
 def _finish_batch(pending):
@@ -329,12 +484,15 @@ def _finish_batch(pending):
     solver, cases, shapes, keep, host, head = pending
     solver.stream.synchronize()
     hd = head.numpy()
-    st = int(hd[:4].view(np.int32)[0])
-    if st != 0:
-        _lib.check(st, "solve_batch")
+    n = len(cases)
+    status = [int(hd[:4].view(np.int32)[0])]
+    if len(hd) > 64 + 16 * n:  # status words of the parts after the first, 64 bytes apart
+        status += hd[64 + 16 * n :].view(np.int32)[::16].tolist()
+    for st in status:
+        if st != 0:
+            _lib.check(st, "solve_batch")
     hn = host.numpy()
     results = BatchResults()
-    n = len(cases)
     if getattr(solver, "check", True):
         results._sums = hd[64 : 64 + 16 * n].view(np.float32).reshape(n, 4).copy()
     if n and all(sh == shapes[0] for sh in shapes):  # one geometry: views of one reshaped array
@@ -413,8 +571,8 @@ def solve_batch(cases, *, solver=None):
     """Solve a list of cases (keyword-argument dicts of
     ``steady_state_transport_solver``) in FP32 on the GPU; returns a list of
     ``(grid, conc, flx)`` with the single-case function's shapes and dtypes.
-    All outputs come back in one device-to-host copy into a fresh pinned
-    buffer that the returned arrays view; the grid arrays are shared
-    read-only arrays."""
+    All outputs come back into one fresh pinned buffer that the returned
+    arrays view, a large batch's in parts that overlap its computation; the
+    grid arrays are shared read-only arrays."""
     solver = solver or BatchSolver()
-    return _finish_batch(_enqueue_batch(solver, cases))
+    return _finish_batch(_enqueue_parts(solver, cases))

@@ -1621,6 +1621,31 @@ int bldfm_memcpy_async(void *dst, const void *src, size_t bytes, void *stream)
                                                                                                  : BLDFM_ERR_CUDA;
 }
 
+int bldfm_upload_async(void *dst, const void *src, size_t bytes, void *stream)
+{
+    return bldfm_guarded([&]() -> int {
+        if (bytes == 0) return BLDFM_OK;
+        if (!dst || !src) return BLDFM_ERR_ARG;
+        std::lock_guard<std::mutex> lk(g_mutex);
+        int status = BLDFM_OK;
+        DeviceCache &dc = cache_for_current(&status);
+        if (status != BLDFM_OK) return status;
+        // 1 MB at a time through the ring of staging buffers: the copy into one
+        // overlaps the transfer of the one before, and the ring stays small
+        const size_t chunk = (size_t)1 << 20;
+        for (size_t o = 0; o < bytes; o += chunk) {
+            const size_t nb = std::min(chunk, bytes - o);
+            StageSlot *slt = nullptr;
+            int rc = acquire_stage(dc, nb, &slt);
+            if (rc != BLDFM_OK) return rc;
+            memcpy(slt->buf, (const char *)src + o, nb);
+            CK(cudaMemcpyAsync((char *)dst + o, slt->buf, nb, cudaMemcpyHostToDevice, (cudaStream_t)stream));
+            CK(cudaEventRecord(slt->ev, (cudaStream_t)stream));
+        }
+        return BLDFM_OK;
+    });
+}
+
 int bldfm_stage_times(float *ms, int n)
 {
     std::lock_guard<std::mutex> lk(g_mutex);

@@ -171,6 +171,12 @@ int bldfm_stage_times(float *ms, int n);
  * buffer with it). */
 int bldfm_memcpy_async(void *dst, const void *src, size_t bytes, void *stream);
 
+/* Copy host data of any kind to the device on the caller's stream through the
+ * library's pinned staging ring: src may be changed or freed as soon as the
+ * call returns.  No reference counterpart (the sources of a batch go up with
+ * it). */
+int bldfm_upload_async(void *dst, const void *src, size_t bytes, void *stream);
+
 /* Algorithmic flops of the FP32 Riccati sweep for one solved mode (an FMA
  * counted as 2, MUL/ADD/RCP as 1) on the nz-level table of prof_host with
  * output levels levels_host: the steps above the highest output level update

@@ -150,3 +150,29 @@ def test_batch_forward_passes(sizes):
         _, oc, of = O.steady_state_transport_solver(**kw)
         assert relerr(c.cpu().numpy() if hasattr(c, "cpu") else c, oc) <= 1e-4
         assert relerr(f.cpu().numpy() if hasattr(f, "cpu") else f, of) <= 1e-4
+
+
+def test_solve_batch_in_parts(monkeypatch):
+    """A batch that goes back in parts gives the bits of the whole batch, with its
+    error statements, status word and refusals."""
+    from bldfm_gb300 import batch as B
+
+    z, p = O.vertical_profiles(8, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    cases = [dict(srf_flx=np.full((ny, nx), 0.5), z=z, profiles=p, domain=(4.0 * nx, 4.0 * ny), levels=lv,
+                  modes=(nx, ny), meas_pt=(3.0, 2.0), footprint=fp, halo=8.0, precision="double")
+             for nx, ny, lv, fp in [(64, 48, 8, True), (40, 30, [0, 8], False), (128, 96, 8, True), (6, 4, 8, False),
+                                    (64, 48, [2, 4, 8], False)]]
+    whole, s = B.solve_batch(cases), B.BatchSolver()
+    monkeypatch.setattr(B, "PART_BYTES", 1 << 16)
+    assert len(B._split_batch([B._output_bound(kw) for kw in cases])) > 2
+    for _ in range(3):
+        got = B.solve_batch(cases, solver=s)
+        assert s.status() == 0
+        # sums of 32 positive FP32 samples added atomically, in any order
+        np.testing.assert_allclose(got.error_estimates, whole.error_estimates, rtol=32 * 2.0**-23)
+        np.testing.assert_array_equal(s.error_estimates(len(cases)), got.error_estimates)
+        for (_, c0, f0), (_, c1, f1) in zip(whole, got):
+            np.testing.assert_array_equal(c0, c1)
+            np.testing.assert_array_equal(f0, f1)
+        with pytest.raises(ValueError):
+            B.solve_batch(cases[:-1] + [dict(cases[-1], modes=(5, 4))], solver=s)
