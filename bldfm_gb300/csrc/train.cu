@@ -746,7 +746,8 @@ __device__ __forceinline__ void write_blocks(const MlpBlocks &k, int j, int e, f
     k.Wb[j][mlp_chunk_index(in, out)] = b;
     k.Wt[j][tc_core_offset(out, in, MLP_H) / 2] = b;
     const int q = (out >> 7) * 2 + (in >> 7);
-    k.Wq[j][(size_t)q * 128 * 128 + tc_core_offset(out & 127, in & 127, 128) / 2] = b;
+    // halved (exact in BF16): the serving kernel's GELU takes z / 2
+    k.Wq[j][(size_t)q * 128 * 128 + tc_core_offset(out & 127, in & 127, 128) / 2] = f2bf(0.5f * w);
 }
 
 // hidden layer (1..3) and element of its weight matrix of parameter i, or 0

@@ -30,7 +30,7 @@ size_t mlp_train_part_o(int batch, int nsm);
 
 // bf16 operand blocks of the hidden weights: Wf (rows out, K in) and Wb (rows
 // in, K out) in K chunks for the training step, Wt (rows out, K in) for the
-// layer-by-layer forward pass, Wq = Wt as four 128 x 128 quarters for serving
+// layer-by-layer forward pass, Wq = Wt / 2 as four 128 x 128 quarters for serving
 struct MlpBlocks {
     uint16_t *Wf[3], *Wb[3], *Wt[3], *Wq[3];
 };

@@ -176,3 +176,23 @@ def test_solve_batch_in_parts(monkeypatch):
             np.testing.assert_array_equal(f0, f1)
         with pytest.raises(ValueError):
             B.solve_batch(cases[:-1] + [dict(cases[-1], modes=(5, 4))], solver=s)
+
+
+@pytest.mark.parametrize("count,size", [(1, 10), (130, 32), (3, 200)])
+def test_serving_tiles(count, size):
+    """The fused serving kernel with fewer tiles than SMs, with a new case at
+    every tile of a block, and with several tiles of a case per block: the batch
+    gives the single footprints (the bar of the batched serving test)."""
+    from bldfm_gb300.surrogate import Surrogate, load
+
+    net, _, _ = load()
+    sur = Surrogate(net, spot_every=0)
+    dom = (3.9 * size, 3.9 * size)
+    items = [dict(n=128, zm=20.0, wind=(3.0 * math.cos(i), 3.0 * math.sin(i)), srf_shape=(size, size), domain=dom,
+                  modes=(size, size), meas_pt=(0.5 * dom[0], 0.4 * dom[1]), ustar=0.3, mol=-50.0 - i)
+             for i in range(count)]
+    outs = [(c.cpu().numpy(), f.cpu().numpy()) for c, f in sur.solve_batch_prepared(sur.prepare_batch(items))]
+    assert sur.status() == 0
+    for i in range(0, count, 13):
+        c, f = sur.solve_prepared(sur.prepare(**items[i]))
+        assert relerr(outs[i][0], c.cpu().numpy()) < 1e-6 and relerr(outs[i][1], f.cpu().numpy()) < 1e-6
