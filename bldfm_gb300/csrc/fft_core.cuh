@@ -145,6 +145,29 @@ __device__ __forceinline__ void dft_small(C *u, const C *tw, int n)
             u[t] = cx_add(a[t], b[t]);
             u[t + 4] = cx_sub(a[t], b[t]);
         }
+    } else if (P == 5 && sizeof(RR) == 8) {
+        // FP64: symmetric inputs folded (36 operations where the direct sums,
+        // whose order FP32 keeps, take 104)
+        const RR c1 = (RR)0.30901699437494742410229341718282, c2 = (RR)-0.80901699437494742410229341718282;
+        const RR s1 = (RR)(sign * 0.95105651629515357211643933337938), s2 = (RR)(sign * 0.58778525229247312916870595463907);
+        const C S1 = cx_add(u[1], u[4]), D1 = cx_sub(u[1], u[4]), S2 = cx_add(u[2], u[3]), D2 = cx_sub(u[2], u[3]);
+        const C a = u[0];
+        C A1, A2, B1, B2;
+        A1.x = fma(c2, S2.x, fma(c1, S1.x, a.x));
+        A1.y = fma(c2, S2.y, fma(c1, S1.y, a.y));
+        A2.x = fma(c1, S2.x, fma(c2, S1.x, a.x));
+        A2.y = fma(c1, S2.y, fma(c2, S1.y, a.y));
+        B1.x = fma(s2, D2.x, s1 * D1.x);
+        B1.y = fma(s2, D2.y, s1 * D1.y);
+        B2.x = fma(-s1, D2.x, s2 * D1.x);
+        B2.y = fma(-s1, D2.y, s2 * D1.y);
+        u[0] = cx_add(a, cx_add(S1, S2));
+        B1 = cx_rot(B1, 1.f);  // i B
+        B2 = cx_rot(B2, 1.f);
+        u[1] = cx_add(A1, B1);
+        u[4] = cx_sub(A1, B1);
+        u[2] = cx_add(A2, B2);
+        u[3] = cx_sub(A2, B2);
     } else if (P == 5) {
         C o[5];
         for (int j = 0; j < 5; ++j) {
