@@ -212,11 +212,12 @@ struct DeviceCache {
     int nsm = 0;
     std::map<int, TwTable> tw;
     std::map<std::pair<int, int>, ModeList> modes;
-    // a second stream per caller stream: the batch's accuracy check runs on
-    // it beside the transform passes (fork and join by events)
+    // two more streams per caller stream (fork and join by events): the batch's
+    // accuracy check runs on one beside the transform passes, the passes of the
+    // smaller groups of line lengths on the other
     struct Aux {
-        cudaStream_t s = nullptr;
-        cudaEvent_t fork = nullptr, join = nullptr;
+        cudaStream_t s = nullptr, s2 = nullptr;
+        cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
     };
     std::map<cudaStream_t, Aux> aux;
     std::map<std::vector<int>, int4 *> xband;
@@ -264,7 +265,9 @@ int get_aux(DeviceCache &dc, cudaStream_t st, DeviceCache::Aux **out)
     if (it == dc.aux.end()) {
         DeviceCache::Aux a;
         if (cudaStreamCreateWithFlags(&a.s, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&a.s2, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&a.fork, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&a.join2, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&a.join, cudaEventDisableTiming) != cudaSuccess)
             return BLDFM_ERR_CUDA;
         it = dc.aux.emplace(st, a).first;
@@ -853,6 +856,7 @@ int batch_build(const bldfm_case *cs, int n, const bldfm_batch_opts *opts, Devic
             B.row0[k] = B.nrow - x.row_start;
             B.ncol += g.nlvls * ((g.nbx + B.cpck[k] - 1) / B.cpck[k]);
             B.nrow += g.nlvls * ((g.out_ny + B.rpck[k] - 1) / B.rpck[k]);
+            x.points += (int64_t)g.nlvls * g.out_ny * g.out_nx;
         }
         x.col_ctas = B.ncol - x.col_start;
         x.row_ctas = B.nrow - x.row_start;
@@ -1166,20 +1170,25 @@ int batch_enqueue(const bldfm_case *cs, int n, BatchBuild &B, char *ws, const vo
     bl.nxg = B.nxg;
     for (int i = 0; i < B.nxg; ++i) bl.xg[i] = B.xg[i];
     if (tdc) tmark(*tdc, st);  // 1: the sweep
-    CK(launch_batch_kernels(bl, st, 0));
+    CK(launch_batch_kernels(bl, st, 0, st));
     if (disp && side) CK(cudaStreamWaitEvent(st, aux->join, 0));
     // the accuracy check reads the spectra, as the transform passes do: it
     // runs beside them on the auxiliary stream (after them when the stages
     // are timed, so that each stage's time is its own)
-    const bool fork = B.check && side;
+    const bool fork = B.check && side, split = side && B.rx_col >= 0 && B.nxg > 1;
+    if (fork || split) CK(cudaEventRecord(aux->fork, st));
     if (fork) {
-        CK(cudaEventRecord(aux->fork, st));
         CK(cudaStreamWaitEvent(aux->s, aux->fork, 0));
         CK(launch_fp32_check(bl.cases, n, (float4 *)(ws + 64), aux->s));
         CK(cudaEventRecord(aux->join, aux->s));
     }
     if (tdc) tmark(*tdc, st);  // 2: the output transform
-    CK(launch_batch_kernels(bl, st, 1));
+    if (split) CK(cudaStreamWaitEvent(aux->s2, aux->fork, 0));
+    CK(launch_batch_kernels(bl, st, 1, split ? aux->s2 : st));
+    if (split) {
+        CK(cudaEventRecord(aux->join2, aux->s2));
+        CK(cudaStreamWaitEvent(st, aux->join2, 0));
+    }
     if (tdc) tmark(*tdc, st);  // 3: the accuracy check
     if (fork)
         CK(cudaStreamWaitEvent(st, aux->join, 0));
@@ -1566,7 +1575,7 @@ int sur_solve_batch_impl(void *net, const bldfm_case *cs, const bldfm_surrogate_
     bl.rx_row = B.rx_row;
     bl.nxg = B.nxg;
     for (int i = 0; i < B.nxg; ++i) bl.xg[i] = B.xg[i];
-    CK(launch_batch_kernels(bl, st, 1));
+    CK(launch_batch_kernels(bl, st, 1, st));
     tmark(dc, st);  // 5: end
     return BLDFM_OK;
 }

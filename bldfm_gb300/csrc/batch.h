@@ -41,6 +41,7 @@ struct __align__(16) BatchCase {
 struct XGroup {
     int rx_col, rx_row;
     int col_start, col_ctas, row_start, row_ctas;
+    int64_t points;  // output points of its cases
 };
 
 struct BatchLaunch {
@@ -66,7 +67,9 @@ struct BatchLaunch {
     XGroup xg[BATCH_MAX_XGROUPS];
 };
 
-cudaError_t launch_batch_kernels(const BatchLaunch &bl, cudaStream_t st, int part);
+// part 0: the sweep; part 1: the transform passes, those of the exact-length
+// groups other than the largest on `side` (may be st)
+cudaError_t launch_batch_kernels(const BatchLaunch &bl, cudaStream_t st, int part, cudaStream_t side);
 
 // Accuracy check of a batched FP32 solve (batch.cu: fp32_check_kernel): a
 // stratified sample of 32 modes per case evaluated in float-float arithmetic
