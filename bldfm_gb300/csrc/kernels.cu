@@ -106,11 +106,24 @@ __device__ __forceinline__ void sweep_item(const SweepItems &s, int nly, int i, 
     m0 = s.C0 + (int64_t)s.F * nly + (j - s.F * s.I);
 }
 
+#define SWEEP64_THREADS 512
+
+// Items of a thread of the FP64 sweeps: warps of 32 items, dealt to the blocks
+// (one per SM) in turn, so that every SM holds the same number to within one.
+struct SweepWarp {
+    int64_t first, step;
+    __device__ __forceinline__ SweepWarp()
+    {
+        first = 32 * ((int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) + (threadIdx.x & 31);
+        step = (int64_t)blockDim.x * gridDim.x;
+    }
+};
+
 // NM modes per thread (2: the items above).  Writes per mode: top states
 // (p1,q1,p2,q2) and the same four states at every snapshot slot.
 //   snap layout: [(slot * 4 + j) * nsolved + m],  top layout: [j * nsolved + m]
 template <int NM>
-__global__ void __launch_bounds__(128) sweep64_kernel(SolveGeom g, const double *__restrict__ lvtab,
+__global__ void __launch_bounds__(SWEEP64_THREADS) sweep64_kernel(SolveGeom g, const double *__restrict__ lvtab,
                                                       const int *__restrict__ slot_of_step,
                                                       const uint32_t *__restrict__ modes,
                                                       const double2 *__restrict__ q0spec,
@@ -135,7 +148,8 @@ __global__ void __launch_bounds__(128) sweep64_kernel(SolveGeom g, const double 
     const int64_t ns = g.nsolved;
     const SweepItems si = sweep_items(g.nlx, g.nly);
     const int64_t n = NM == 2 ? si.n : ns;
-    for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it < n; it += (int64_t)gridDim.x * blockDim.x) {
+    const SweepWarp sw;
+    for (int64_t it = sw.first; it < n; it += sw.step) {
         int r, c;
         int64_t m[2] = {it, -1};
         if (NM == 2) {
@@ -491,7 +505,7 @@ struct RiccState {
 };
 
 template <bool SINGLE, int NM>
-__global__ void __launch_bounds__(128) riccati64_kernel(SolveGeom g, const double *__restrict__ lvtab,
+__global__ void __launch_bounds__(SWEEP64_THREADS) riccati64_kernel(SolveGeom g, const double *__restrict__ lvtab,
                                                         const int *__restrict__ slot_of_step,
                                                         const uint32_t *__restrict__ modes,
                                                         const double2 *__restrict__ q0spec,
@@ -524,7 +538,8 @@ __global__ void __launch_bounds__(128) riccati64_kernel(SolveGeom g, const doubl
     const int64_t ns = g.nsolved;
     const SweepItems si = sweep_items(g.nlx, g.nly);
     const int64_t n = NM == 2 ? si.n : ns;
-    for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it < n; it += (int64_t)gridDim.x * blockDim.x) {
+    const SweepWarp sw;
+    for (int64_t it = sw.first; it < n; it += sw.step) {
         int r, c;
         int64_t m[2] = {it, -1};
         if (NM == 2) {
@@ -689,32 +704,34 @@ __global__ void __launch_bounds__(128) riccati64_kernel(SolveGeom g, const doubl
     }
 }
 
-// Modes per thread and threads per block of the FP64 sweeps.  The pipe passes
-// one instruction per 16 clocks and SM, but of one warp only one per 64, so a
-// launch takes (warps of the fullest SM, at least 4) x (instructions of a
-// warp): one1 for a warp of single modes, one2 of pairs.  Pairs issue fewer in
-// all but come in coarser units, and reach 95% of the pipe's rate (single modes
-// 99%): 128^2 modes over 47 levels take 106 us as singles, 191 us as pairs,
-// 384^2 modes 885 and 821.  Small blocks spread a small solve evenly (256^2
-// modes: 772 us in blocks of one warp, 877 in blocks of four), larger ones
-// where the level table leaves room for few.
+// Launch of the FP64 sweeps.  The pipe passes one instruction per 16 clocks and
+// SM, but of one warp only one per 64, so a launch takes (warps of the fullest
+// SM, at least 4) x (instructions of a warp): one1 for a warp of single modes,
+// one2 of pairs.  Pairs issue fewer in all but come in coarser units, and reach
+// 95% of the pipe's rate (single modes 99%): 128^2 modes over 47 levels take 106
+// us as singles, 191 us as pairs, 384^2 modes 885 and 821.  One block per SM
+// holds all its warps, at most 16: the number per SM is exact (small blocks are
+// not dealt evenly), they share a level table, and more work goes in rounds of
+// equal size, as a last round of fewer than four warps runs at their own rate.
+// 512^2 modes over 207 levels: 3035 us in blocks of one warp, 2858 so (97% of
+// the pipe for 14 warps an SM); the accurate sweep of 512^2 over 104: 869, 805.
 struct Sweep64Launch {
     bool pairs;
     int threads;
     unsigned blocks;
 };
 
-static Sweep64Launch sweep64_launch(const SolveGeom &g, size_t smem, int nsm, double one1, double one2)
+static Sweep64Launch sweep64_launch(const SolveGeom &g, int nsm, double one1, double one2)
 {
+    auto per_sm = [&](int64_t n) { return ((n + 31) / 32 + nsm - 1) / nsm; };
+    auto units = [&](int64_t n) { return (double)std::max<int64_t>(per_sm(n), 4); };
     const int64_t n2 = sweep_items(g.nlx, g.nly).n;
-    auto units = [&](int64_t n) { return (double)std::max<int64_t>(((n + 31) / 32 + nsm - 1) / nsm, 4); };
     Sweep64Launch l;
     l.pairs = units(n2) * one2 < 0.95 * units(g.nsolved) * one1;
-    const int64_t n = l.pairs ? n2 : g.nsolved;
-    const int fit = (int)((227 * 1024) / (smem + 1024));  // blocks per SM
-    l.threads = fit >= 8 ? 32 : fit >= 4 ? 64 : 128;
-    int64_t b = (n + l.threads - 1) / l.threads;
-    l.blocks = (unsigned)std::min<int64_t>(std::max<int64_t>(b, 1), 256LL * nsm);
+    const int64_t n = l.pairs ? n2 : g.nsolved, w = per_sm(n);
+    const int64_t rounds = (w + SWEEP64_THREADS / 32 - 1) / (SWEEP64_THREADS / 32);
+    l.threads = 32 * (int)((w + rounds - 1) / rounds);
+    l.blocks = (unsigned)std::min<int64_t>((n + 31) / 32, nsm);
     return l;
 }
 
@@ -724,7 +741,7 @@ cudaError_t launch_riccati64(const SolveGeom &g, const double *lvtab, const int 
     if (g.nsnap < 1 || g.nsolved == 0) return cudaSuccess;
     const size_t smem = (size_t)(g.nz - 1) * RT_N * sizeof(double) + (size_t)g.nz * sizeof(int) + 16;
     const double above = g.nz - 1 - g.jmax, below = g.jmax;
-    const Sweep64Launch l = sweep64_launch(g, smem, nsm, above * 30 + below * 40, above * 54 + below * 73);
+    const Sweep64Launch l = sweep64_launch(g, nsm, above * 30 + below * 40, above * 54 + below * 73);
     auto run = [&](auto k) { k<<<l.blocks, l.threads, smem, st>>>(g, lvtab, slot, modes, q0spec, scratch, Xp, Xq); };
     if (g.nsnap == 1)
         l.pairs ? run(riccati64_kernel<true, 2>) : run(riccati64_kernel<true, 1>);
@@ -944,7 +961,7 @@ cudaError_t launch_sweep64(const SolveGeom &g, const double *lvtab, const int *s
         cudaFuncSetAttribute(sweep64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(sweep64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     }
-    const Sweep64Launch l = sweep64_launch(g, smem, nsm, 68, 124);
+    const Sweep64Launch l = sweep64_launch(g, nsm, 68, 124);
     if (l.pairs)
         sweep64_kernel<2><<<l.blocks, l.threads, smem, st>>>(g, lvtab, slot, modes, q0spec, snap, top, err);
     else
