@@ -53,6 +53,8 @@ __device__ __forceinline__ void tc_fence_init()
 }
 
 // Bounded wait for phase `parity` of an mbarrier; false if the limit ran out.
+// The wait suspends between tries: polling takes issue and memory-queue slots
+// from the warps that compute (the training step 147 us against 144).
 __device__ __forceinline__ bool tc_mbar_wait(uint64_t *bar, uint32_t parity)
 {
     const uint32_t a = tc_smem(bar);
@@ -68,26 +70,6 @@ __device__ __forceinline__ bool tc_mbar_wait(uint64_t *bar, uint32_t parity)
         if (done) return true;
     }
     return false;
-}
-
-// Bounded wait for an event that is near: polls first (a suspended wait takes
-// about 2 us to return, longer than the copy or MMA it waits for), then
-// suspends as tc_mbar_wait does.
-__device__ __forceinline__ bool tc_poll_wait(uint64_t *bar, uint32_t parity)
-{
-    const uint32_t b = tc_smem(bar);
-    for (int it = 0; it < 4096; ++it) {
-        uint32_t d;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(d)
-            : "r"(b), "r"(parity)
-            : "memory");
-        if (d) return true;
-    }
-    return tc_mbar_wait(bar, parity);
 }
 
 // named barrier of n threads

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
 #pragma unroll 1
                 for (int c2 = 0; c2 < 2 * NCHUNK; ++c2, ++q) {
                     const int c = c2 % NCHUNK, s = (int)(q % RING);
-                    if (q >= RING) ok = tc_poll_wait(&empty[s], (q / RING - 1) & 1);
+                    if (q >= RING) ok = tc_mbar_wait(&empty[s], (q / RING - 1) & 1);
                     if (!ok) break;
                     tc_load_warp(smem + OFF_RING + s * CHUNK_BYTES, w + (size_t)c * MLP_H * MLP_KC, CHUNK_BYTES,
                                  CHUNK_BYTES, &full[s]);
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
             for (int g = 0; g < NGEMM && ok; ++g, ++nready) {
 #pragma unroll 1
                 for (int t = 0; t < 2 && ok; ++t) {
-                    ok = tc_poll_wait(&ready[t], nready & 1);
+                    ok = tc_mbar_wait(&ready[t], nready & 1);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t da = tc_desc(tc_smem(smem + t * TILE_BYTES), 128, (MLP_H / 8) * 128);
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
 #pragma unroll 1
                     for (int c = 0; c < NCHUNK; ++c, ++q) {
                         const int s = (int)(q % RING);
-                        ok = tc_poll_wait(&full[s], (q / RING) & 1);
+                        ok = tc_mbar_wait(&full[s], (q / RING) & 1);
                         if (!ok) break;
                         tc_fence_after();
                         const uint64_t db = tc_desc(tc_smem(smem + OFF_RING + s * CHUNK_BYTES), 128, (MLP_KC / 8) * 128);
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) mlp_step_kernel(const StepArg
         };
         auto take = [&]() -> bool {
             // the tile's threads agree, so that none waits for one that gave up
-            if (!tc_bar_and(bar_tile, 256, tc_poll_wait(&done[t], ngemm & 1))) return false;
+            if (!tc_bar_and(bar_tile, 256, tc_mbar_wait(&done[t], ngemm & 1))) return false;
             ++ngemm;
             tc_fence_after();
             return true;
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) mlp_grad_kernel(const GradArg
 #pragma unroll 1
         for (; i < n; ++i) {
             const int st = i % GSTAGES;
-            if (!(ok = tc_poll_wait(&full[st], (uint32_t)(i / GSTAGES) & 1))) break;
+            if (!(ok = tc_mbar_wait(&full[st], (uint32_t)(i / GSTAGES) & 1))) break;
             tc_fence_after();
             const uint32_t a0 = tc_smem(smem + st * (GA_BYTES + GB_BYTES));
             // MN-major, no swizzle: 8-feature groups 128 bytes apart (the
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) mlp_grad_kernel(const GradArg
             tc_commit_warp(&empty[st]);
             if (i > 0 && loaded < n) {
                 const int p = i - 1;
-                if (!(ok = tc_poll_wait(&empty[p % GSTAGES], (uint32_t)(p / GSTAGES) & 1))) break;
+                if (!(ok = tc_mbar_wait(&empty[p % GSTAGES], (uint32_t)(p / GSTAGES) & 1))) break;
                 load(loaded++);
             }
         }
