@@ -1547,10 +1547,21 @@ int sur_solve_batch_impl(void *net, const bldfm_case *cs, const bldfm_surrogate_
     CK(launch_sur_lowband((const LowBandCase *)(wb + B.extra_off + sur_lowband_off(n)), n, lb_total, lb_maxnz, st));
     tmark(dc, st);  // 3: the accuracy guard
     float4 *acc = (float4 *)(w + B.total);
-    CK(cudaMemsetAsync(acc, 0, 16 * (size_t)n, st));
+    // the guard reads the spectra, as the transform passes do: beside them on
+    // the auxiliary stream, before them when the stages are timed
+    const bool fork = !dc.timing;
+    DeviceCache::Aux *aux = nullptr;
+    if (fork) {
+        if ((rc = get_aux(dc, st, &aux)) != BLDFM_OK) return rc;
+        CK(cudaEventRecord(aux->fork, st));
+        CK(cudaStreamWaitEvent(aux->s, aux->fork, 0));
+    }
+    const cudaStream_t gs = fork ? aux->s : st;
+    CK(cudaMemsetAsync(acc, 0, 16 * (size_t)n, gs));
     CK(launch_sur_guard((const BatchCase *)(wb + B.off_cases), n,
                         (const int64_t *)(wb + B.extra_off + sur_prefix_off(n)), prefix[n], SUR_GUARD_STRIDE, lb_maxnz,
-                        acc, st));
+                        acc, gs));
+    if (fork) CK(cudaEventRecord(aux->join, gs));
     tmark(dc, st);  // 4: the output transform
     BatchLaunch bl;
     memset(&bl, 0, sizeof(bl));
@@ -1576,6 +1587,7 @@ int sur_solve_batch_impl(void *net, const bldfm_case *cs, const bldfm_surrogate_
     bl.nxg = B.nxg;
     for (int i = 0; i < B.nxg; ++i) bl.xg[i] = B.xg[i];
     CK(launch_batch_kernels(bl, st, 1, st));
+    if (fork) CK(cudaStreamWaitEvent(st, aux->join, 0));
     tmark(dc, st);  // 5: end
     return BLDFM_OK;
 }
