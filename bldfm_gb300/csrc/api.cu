@@ -1524,6 +1524,9 @@ int sur_solve_batch_impl(void *net, const bldfm_case *cs, const bldfm_surrogate_
         const int nb = sur_lowband_setup(c, mets[k].exact_kz, mets[k].zm);
         if (nb > INT_MAX - lb_total) return BLDFM_ERR_ARG;
         lb_total += nb;
+        sc[k].band_kmax2 = c.count > 0 ? c.kmax2 : 0.f;
+        sc[k].band_bx = c.ncol > 0 ? c.g.nlx / 2 : c.bx;
+        sc[k].band_by = c.nrow > 0 ? c.g.nly / 2 : c.by;
         lb_maxnz = std::max(lb_maxnz, c.g.nz);
     }
     int64_t *prefix = (int64_t *)(blob + B.extra_off + sur_prefix_off(n));
@@ -1542,26 +1545,35 @@ int sur_solve_batch_impl(void *net, const bldfm_case *cs, const bldfm_surrogate_
     if ((rc = mlp_serving_view(net, &view)) != BLDFM_OK) return rc;
     char *wb = w + B.blob_at;
     tmark(dc, st);  // 1: the fused features -> MLP -> spectra kernel
-    CK(launch_sur_serve((const SurCase *)(wb + B.extra_off), n, t, view, (int *)w, dc.nsm, st));
-    tmark(dc, st);  // 2: the exact low band
-    CK(launch_sur_lowband((const LowBandCase *)(wb + B.extra_off + sur_lowband_off(n)), n, lb_total, lb_maxnz, st));
-    tmark(dc, st);  // 3: the accuracy guard
-    float4 *acc = (float4 *)(w + B.total);
-    // the guard reads the spectra, as the transform passes do: beside them on
-    // the auxiliary stream, before them when the stages are timed
+    // The exact low band beside the network on the auxiliary stream (they write
+    // different modes), then the guard, which reads the spectra as the
+    // transform passes do, beside those; one after another when the stages are
+    // timed.  The network's blocks leave room for some of the band's on every SM.
     const bool fork = !dc.timing;
     DeviceCache::Aux *aux = nullptr;
+    cudaStream_t as = st;
     if (fork) {
         if ((rc = get_aux(dc, st, &aux)) != BLDFM_OK) return rc;
+        as = aux->s;
         CK(cudaEventRecord(aux->fork, st));
-        CK(cudaStreamWaitEvent(aux->s, aux->fork, 0));
     }
-    const cudaStream_t gs = fork ? aux->s : st;
-    CK(cudaMemsetAsync(acc, 0, 16 * (size_t)n, gs));
+    CK(launch_sur_serve((const SurCase *)(wb + B.extra_off), n, t, view, (int *)w, dc.nsm, st));
+    tmark(dc, st);  // 2: the exact low band
+    if (fork) CK(cudaStreamWaitEvent(as, aux->fork, 0));
+    float4 *acc = (float4 *)(w + B.total);
+    CK(cudaMemsetAsync(acc, 0, 16 * (size_t)n, as));
+    CK(launch_sur_lowband((const LowBandCase *)(wb + B.extra_off + sur_lowband_off(n)), n, lb_total, lb_maxnz, as));
+    if (fork) {
+        CK(cudaEventRecord(aux->join, as));
+        CK(cudaStreamWaitEvent(st, aux->join, 0));
+        CK(cudaEventRecord(aux->fork, st));
+        CK(cudaStreamWaitEvent(as, aux->fork, 0));
+    }
+    tmark(dc, st);  // 3: the accuracy guard
     CK(launch_sur_guard((const BatchCase *)(wb + B.off_cases), n,
                         (const int64_t *)(wb + B.extra_off + sur_prefix_off(n)), prefix[n], SUR_GUARD_STRIDE, lb_maxnz,
-                        acc, gs));
-    if (fork) CK(cudaEventRecord(aux->join, gs));
+                        acc, as));
+    if (fork) CK(cudaEventRecord(aux->join, as));
     tmark(dc, st);  // 4: the output transform
     BatchLaunch bl;
     memset(&bl, 0, sizeof(bl));

@@ -95,9 +95,10 @@ cudaError_t launch_sur_guard(const BatchCase *cases, int n, const int64_t *prefi
 // transform.  The band's modes are enumerated over the half box kx in
 // [0, bx], ky in [-by, by] (kx = 0: ky in [1, by]), then, when the box
 // reaches an even mode count's Nyquist frequency, the unpaired modes of the
-// Nyquist column kx = -nlx/2 and row ky = -nly/2; two per thread, 512 per
-// CTA; modes outside the disc are skipped.
-#define SUR_LOWBAND_THREADS 256
+// Nyquist column kx = -nlx/2 and row ky = -nly/2; two per thread, 128 per
+// CTA; modes outside the disc are skipped.  CTAs of two warps fit beside the
+// network's on an SM (alone, eight warps a CTA would be 4% faster).
+#define SUR_LOWBAND_THREADS 64
 #define SUR_LOWBAND_MODES (2 * SUR_LOWBAND_THREADS)  // box positions per CTA
 struct __align__(16) LowBandCase {
     SolveGeom g;

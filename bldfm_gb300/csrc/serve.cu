@@ -109,9 +109,12 @@ __global__ void sur_spectra_kernel(const SolveGeom g, const uint32_t *__restrict
 #define SV_WARPS 16  // epilogue warps: 4 per TMEM lane quarter, each 2 x 16 columns of a half
 #define SV_OUT_GROUPS 2  // column groups of the output layer's partial sums
 #define SV_ROWS 64  // threads of the two row warps (features, spectra), two rows each
-// + one control warp (copies and MMAs): 19 warps, five a scheduler, which leaves
-// 96 registers a thread (a sixth would leave 80)
+// + one control warp (copies and MMAs): 19 warps, five a scheduler, which would
+// leave 96 registers a thread.  At 88 two warps of the exact low band's kernel
+// fit beside them on every SM (16 footprints of 512^2: network 861 us and band
+// 115 after it; 890 with the band, 695, inside).
 #define SV_THREADS (32 * SV_WARPS + 32 + SV_ROWS)
+#define SV_REGS 88
 #define SV_AB(i) (256u + 64u * (uint32_t)(i))  // TMEM column of activation K-half buffer i
 
 struct SvSmem {
@@ -182,6 +185,18 @@ __device__ __forceinline__ void sv_arrive(uint64_t *bar)
 // barrier of the row warps; true if all of them pass true
 __device__ __forceinline__ bool sv_row_sync(bool ok) { return tc_bar_and(2, SV_ROWS, ok); }
 
+// true for a mode that the exact low band writes (lowband_mode's enumeration
+// and its disc, operation for operation)
+__device__ __forceinline__ bool sv_in_band(const SurCase &c, uint32_t e)
+{
+    int r, col;
+    bool paired;
+    unpack_mode(e, r, col, paired);
+    const int kx = freq_of_index(col, c.g.nlx), ky = freq_of_index(r, c.g.nly);
+    const float lx = c.ax * (float)kx, ly = c.ay * (float)ky;
+    return abs(kx) <= c.band_bx && abs(ky) <= c.band_by && fmaf(lx, lx, ly * ly) < c.band_kmax2;
+}
+
 // mode word of row r of a tile (0 past the case's last mode)
 __device__ __forceinline__ uint32_t sv_mode_word(const SurCase &c, int64_t tile, int r)
 {
@@ -244,25 +259,25 @@ __device__ __forceinline__ void sv_gelu32(float *v, const float *bias)
 // ... and its part of the 256 -> 4 output layer: y += v . W4 rows
 __device__ __forceinline__ void sv_out32(const float *v, const float4 *w, const float *W4, float4 &y)
 {
-    // w: the first 8 columns' weights, read before the wait for y; each
-    // further 8 are read one group ahead of the chain
+    // w: the first 4 columns' weights, read before the wait for y; each
+    // further 4 are read one group ahead of the chain
     float2 y01 = make_float2(y.x, y.y), y23 = make_float2(y.z, y.w);
-    float4 wa[8], wb[8];
+    float4 wa[4], wb[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) wa[i] = w[i];
+    for (int i = 0; i < 4; ++i) wa[i] = w[i];
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        if (g < 3)
+    for (int g = 0; g < 8; ++g) {
+        if (g < 7)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) wb[i] = *(const float4 *)&W4[(8 * (g + 1) + i) * MLP_OUT];
+            for (int i = 0; i < 4; ++i) wb[i] = *(const float4 *)&W4[(4 * (g + 1) + i) * MLP_OUT];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float h = v[8 * g + i];
+        for (int i = 0; i < 4; ++i) {
+            const float h = v[4 * g + i];
             y01 = __ffma2_rn(make_float2(h, h), make_float2(wa[i].x, wa[i].y), y01);
             y23 = __ffma2_rn(make_float2(h, h), make_float2(wa[i].z, wa[i].w), y23);
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) wa[i] = wb[i];
+        for (int i = 0; i < 4; ++i) wa[i] = wb[i];
     }
     y = make_float4(y01.x, y01.y, y23.x, y23.y);
 }
@@ -295,8 +310,8 @@ __device__ __forceinline__ void sv_out32(const float *v, const float4 *w, const 
 // spectra beside the layers.
 //
 // What bounds it, in clocks of a tile's 15,300 (16 footprints of 512^2, 109
-// tiles an SM, 861 us; 1003 with 8 epilogue warps, features and spectra on
-// four of them and the MMAs issued from one lane): eight epilogues of a half,
+// tiles an SM, 861 us alone with 96 registers; 1003 with 8 epilogue warps,
+// features and spectra on four of them and the MMAs issued from one lane): eight epilogues of a half,
 // 1,330 each, where tanh.approx takes 1,088 and the FP32 register ports some
 // 1,000; a bubble of 500 to 600 per layer from the end of the half-1 epilogue
 // until the last four MMAs of half 0 have completed; and the output layer,
@@ -307,7 +322,7 @@ __device__ __forceinline__ void sv_out32(const float *v, const float4 *w, const 
 // Every wait is bounded; on a timeout the kernel records BLDFM_ERR_TIMEOUT, all
 // warps leave their loops, the control warp waits (bounded) for its copies and
 // MMAs in flight, and TMEM is freed.
-__global__ void __launch_bounds__(SV_THREADS, 1)
+__global__ void __maxnreg__(SV_REGS)
     sur_serve_kernel(const SurCase *__restrict__ cases, int ncases, int64_t ntiles, const MlpServing net, int *err)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -535,9 +550,9 @@ __global__ void __launch_bounds__(SV_THREADS, 1)
                 if (lane == 0) sv_arrive(&bar_e[h]);
                 sv_gelu32(v, S.bias[3] + 128 * h + 32 * cg);
                 const float *w4 = S.W4 + (128 * h + 32 * cg) * MLP_OUT;
-                float4 w0[8];
+                float4 w0[4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) w0[i] = *(const float4 *)&w4[i * MLP_OUT];
+                for (int i = 0; i < 4; ++i) w0[i] = *(const float4 *)&w4[i * MLP_OUT];
                 // step 2 h + second of the chain: after the one before, the
                 // first when the sums of the tile before last have been read
                 float4 &Yp = S.Yp[par][chain][row];
@@ -627,7 +642,7 @@ __global__ void __launch_bounds__(SV_THREADS, 1)
                 const int rr = rt + u * SV_ROWS;
                 const int64_t m = (tile - c.tile0) * 128 + rr;
                 const float4 a = S.Yp[par][0][rr], b = S.Yp[par][1][rr];
-                if (m < c.g.nsolved) {
+                if (m < c.g.nsolved && !sv_in_band(c, u == 0 ? mw[0] : mw[1])) {
                     const float y[4] = {(a.x + b.x) + S.b4[0], (a.y + b.y) + S.b4[1], (a.z + b.z) + S.b4[2],
                                         (a.w + b.w) + S.b4[3]};
                     emit_spectrum(c.g, u == 0 ? mw[0] : mw[1], y, c.ax, c.ay, c.zm, c.inv_wind, c.ktop, c.utop, c.Xp,

@@ -21,7 +21,9 @@ struct __align__(16) SurCase {
     float ax, ay;                  // wavenumber scales (Lx = ax * kx)
     float zm, s1, s2, s3;          // z_m, z_m / L, ln(z_m / z0), u* / U
     float inv_wind, ktop, utop;    // 1 / U, K~ and U~ of the top level
-    float pad;
+    float band_kmax2;              // modes left to the exact low band: |kx| <= bx, |ky| <= by and
+    int band_bx, band_by;          //   Lx^2 + Ly^2 < kmax2 (0: none)
+    int pad;
     int64_t tile0;                 // first 128-mode tile of this case in the launch
 };
 
