@@ -210,7 +210,7 @@ __device__ __forceinline__ bool block_wait(uint64_t *bar, uint32_t parity)
 // buffers (mbarrier per buffer, bounded waits); the case and its twiddles are
 // loaded when the case changes.  Cases whose arrays do not allow 16-byte
 // copies take out_col_lines, one line per item.  smem: 3 maxn + 4 maxnly complex.
-__global__ void __launch_bounds__(256) out_cols_persist_kernel(const BatchCase *__restrict__ cases,
+__global__ void __launch_bounds__(256, 4) out_cols_persist_kernel(const BatchCase *__restrict__ cases,
                                                                const int *__restrict__ col_case, int nitems, int maxn,
                                                                int maxnly, int *err)
 {
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) out_cols_persist_kernel(const BatchCase *
 // the next row's band values into registers while it transforms the current
 // one; the case and its twiddles are loaded when the case changes.
 // smem: 3 maxn complex.
-__global__ void __launch_bounds__(256) out_rows_persist_kernel(const BatchCase *__restrict__ cases,
+__global__ void __launch_bounds__(256, 4) out_rows_persist_kernel(const BatchCase *__restrict__ cases,
                                                                const int *__restrict__ row_case, int nitems, int maxn,
                                                                int *err)
 {

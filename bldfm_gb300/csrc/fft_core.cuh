@@ -211,6 +211,78 @@ __device__ void stage_p(const C *__restrict__ src, C *__restrict__ dst, int n, i
     }
 }
 
+// Direct sums of a generic stage, inputs twiddled: outputs a .. a + m - 1 (mod
+// p) of bl butterflies, U outputs of U butterflies per thread.
+template <typename C, int SIGN, int U>
+__device__ __forceinline__ void generic_sums(const C *__restrict__ src, C *__restrict__ dst, int n, int bl, int L1,
+                                             int p, int rq, const FDiv drq, const FDiv dnb, const C *__restrict__ tw,
+                                             int a, int m)
+{
+    const int nb = n / p, bh = (bl + U - 1) / U, mh = (m + U - 1) / U;
+    for (int b = threadIdx.x; b < bh * mh; b += blockDim.x) {
+        const int jh = b / bh, b0 = b - jh * bh;
+        bool on_b[U], on_j[U];  // the last thread of an odd count repeats its first
+        int j2[U], step[U], at[U], out[U];  // at: j2 t n / p mod n
+        const C *s[U];
+        C acc[U][U];
+#pragma unroll
+        for (int v = 0; v < U; ++v) {
+            on_j[v] = U * jh + v < m;
+            j2[v] = a + U * jh + (on_j[v] ? v : 0);
+            if (j2[v] >= p) j2[v] -= p;
+            step[v] = j2[v] * nb;
+            at[v] = 0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            on_b[u] = b0 + u * bh < bl;
+            const int bb = b0 + (on_b[u] ? u * bh : 0);
+            const int line = (int)fdiv((uint32_t)bb, dnb);
+            const int loc = bb - line * nb;
+            const int j1 = (int)fdiv((uint32_t)loc, drq);
+            const int k = loc - j1 * rq;
+            s[u] = src + (size_t)line * n + j1 * rq * p + k;
+            out[u] = line * n + j1 * rq + k;
+#pragma unroll
+            for (int v = 0; v < U; ++v) acc[u][v] = s[u][0];
+        }
+#pragma unroll (U == 1 ? 4 : 2)
+        for (int t = 1; t < p; ++t) {
+            C x[U], w[U];
+#pragma unroll
+            for (int v = 0; v < U; ++v) {
+                at[v] += step[v];
+                if (at[v] >= n) at[v] -= n;
+                w[v] = tw_get<C, SIGN>(tw, at[v]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                s[u] += rq;
+                x[u] = *s[u];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < U; ++v) acc[u][v] = cx_add(acc[u][v], cx_mul(x[u], w[v]));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int v = 0; v < U; ++v)
+                if (on_b[u] && on_j[v]) dst[out[u] + L1 * j2[v] * rq] = acc[u][v];
+    }
+}
+
+// the one-by-one form, out of line: both forms inlined would raise the kernels'
+// registers (the persistent row pass from 64 to 128)
+template <typename C, int SIGN>
+__device__ __noinline__ void generic_sums_1(const C *__restrict__ src, C *__restrict__ dst, int n, int bl, int L1,
+                                            int p, int rq, const FDiv drq, const FDiv dnb, const C *__restrict__ tw,
+                                            int a, int m)
+{
+    generic_sums<C, SIGN, 1>(src, dst, n, bl, L1, p, rq, drq, dnb, tw, a, m);
+}
+
 // Generic radix p (a prime >= 7, in practice a large factor of a ragged grid),
 // O(p) work per output, every output its own thread's: a butterfly's p^2
 // products are spread over the block (one thread per butterfly left 2 of 256
@@ -297,22 +369,15 @@ __device__ void stage_generic(C *__restrict__ src, C *__restrict__ dst, int n, i
             }
             __syncthreads();
         }
-        for (int b = threadIdx.x; b < bl * m; b += blockDim.x) {
-            const int j0 = b / bl, bb = b - j0 * bl, j2 = a + j0 < p ? a + j0 : a + j0 - p;
-            const int line = (int)fdiv((uint32_t)bb, dnb);
-            const int loc = bb - line * nb;
-            const int j1 = (int)fdiv((uint32_t)loc, drq);
-            const int k = loc - j1 * rq;
-            const C *s = src + (size_t)line * n + j1 * rq * p + k;
-            C acc = s[0];
-            int jt = 0;  // j2 t mod p
-            for (int t = 1; t < p; ++t) {
-                jt += j2;
-                if (jt >= p) jt -= p;
-                acc = cx_add(acc, cx_mul(s[t * rq], tw_get<C, SIGN>(tw, jt * np_)));
-            }
-            dst[(size_t)line * n + (j1 + L1 * j2) * rq + k] = acc;
-        }
+        // two outputs of two butterflies per thread take four shared-memory
+        // reads for four products where one output takes two reads a product
+        // (the reads bound the stage: 7 fields 422 x 462, lines 1346 = 2 x 673 and
+        // 1386, row pass 464 -> 346 us), where that leaves threads enough busy (73 x
+        // 247, lines 567 and 741: 40 us so, 32 one by one)
+        if (4 * bl * m >= 3 * (int)blockDim.x)
+            generic_sums<C, SIGN, 2>(src, dst, n, bl, L1, p, rq, drq, dnb, tw, a, m);
+        else
+            generic_sums_1<C, SIGN>(src, dst, n, bl, L1, p, rq, drq, dnb, tw, a, m);
     }
 }
 
