@@ -222,6 +222,75 @@ __global__ void __launch_bounds__(SWEEP64_THREADS) sweep64_kernel(SolveGeom g, c
     }
 }
 
+// The sweep of a small solve, which leaves the SMs with fewer than four warps:
+// four lanes per mode, lane 2 k + 0 / 1 for the p / q of shooting state k, so
+// that a lane's chain is 33 instructions a step instead of 68 (every operation
+// and rounding of sweep64_kernel's, B = b or -c).  96^2 modes over 104 levels:
+// 230 us with a mode per thread, 138 so.
+__global__ void __launch_bounds__(SWEEP64_THREADS) sweep64_lanes_kernel(SolveGeom g, const double *__restrict__ lvtab,
+                                                                        const int *__restrict__ slot_of_step,
+                                                                        const uint32_t *__restrict__ modes,
+                                                                        const double2 *__restrict__ q0spec,
+                                                                        double2 *__restrict__ snap,
+                                                                        double2 *__restrict__ top, int *err)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ uint64_t bar;
+    __shared__ double s_one[4];
+    double *s_lv = (double *)smem_raw;
+    const int L = g.nz - 1;
+    int *s_slot = (int *)(s_lv + (size_t)L * BLDFM_LV64);
+    if (threadIdx.x < 4) s_one[threadIdx.x] = threadIdx.x < 2 ? 1.0 : -0.0;
+    if (L > 0) {
+        if (!bulk_load_to_smem(s_lv, lvtab, (uint32_t)((size_t)L * BLDFM_LV64 * sizeof(double)), &bar, err))
+            return;
+    }
+    for (int i = threadIdx.x; i < g.nz; i += blockDim.x) s_slot[i] = slot_of_step[i];
+    __syncthreads();
+    const FmaArith F = {s_one[threadIdx.x & 1], s_one[2 + (threadIdx.x & 1)], 0.0};
+
+    const int64_t ns = g.nsolved;
+    const SweepWarp sw;
+    const int lane = threadIdx.x & 31, part = lane & 3;  // p1, q1, p2, q2
+    const bool isq = part & 1;
+    for (int64_t it = sw.first; it - lane < 4 * ns; it += sw.step) {  // whole warps: the lanes exchange p and q
+        const bool on = it < 4 * ns;
+        const int64_t m = on ? it >> 2 : ns - 1;
+        int r, c;
+        bool paired;
+        unpack_mode(modes[m], r, c, paired);
+        const double lx = wavenumber(freq_of_index(c, g.nlx), g.valx, g.lx_scale);
+        const double ly = wavenumber(freq_of_index(r, g.nly), g.valy, g.ly_scale);
+        const double lx2 = __dmul_rn(lx, lx), ly2 = __dmul_rn(ly, ly);
+        double2 x = make_double2(part == 0 ? 1.0 : 0.0, 0.0);
+        if (part == 3) x = q0spec ? q0spec[(size_t)c * g.nly + r] : make_double2(g.q0dc_fp, 0.0);
+        for (int i = 0; i < L; ++i) {
+            const int s = s_slot[i];
+            if (s >= 0 && on) snap[((size_t)s * 4 + part) * ns + m] = x;
+            const double *lv = s_lv + (size_t)i * BLDFM_LV64;
+            const double tx = F.add(F.mul(lv[LV_KX], lx2), F.mul(lv[LV_KY], ly2));
+            const double ty = F.add(F.mul(lv[LV_U], lx), F.mul(lv[LV_V], ly));
+            const double2 a = make_double2(F.add(F.mul(F.mul(lv[LV_S1], tx), lv[LV_H2]), F.one),
+                                           F.mul(F.mul(lv[LV_S1], ty), lv[LV_H2]));
+            const double2 T2 = F.cmul(make_double2(tx, ty), make_double2(tx, ty));
+            const double k = isq ? lv[LV_S4] : lv[LV_S2];
+            const double vx = F.mul(tx, lv[LV_H]), vy = F.mul(ty, lv[LV_H]);
+            double2 b = make_double2(
+                F.add(F.mul(F.mul(k, isq ? T2.x : tx), lv[LV_H3]), isq ? vx : lv[LV_S3]),
+                F.add(F.mul(F.mul(k, isq ? T2.y : ty), lv[LV_H3]), isq ? vy : F.mz));
+            if (isq) b = make_double2(-b.x, -b.y);
+            double2 o;
+            o.x = __shfl_xor_sync(0xffffffffu, x.x, 1);
+            o.y = __shfl_xor_sync(0xffffffffu, x.y, 1);
+            x = F.cadd(F.cmul(a, x), F.cmul(b, o));
+        }
+        if (!on) continue;
+        const int s = s_slot[g.nz - 1];
+        if (s >= 0) snap[((size_t)s * 4 + part) * ns + m] = x;
+        top[part * ns + m] = x;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // FP64 combination: alpha, levels, complex64 rounding, phase shift, mirror
 // ---------------------------------------------------------------------------
@@ -709,26 +778,29 @@ __global__ void __launch_bounds__(SWEEP64_THREADS) riccati64_kernel(SolveGeom g,
 // SM, at least 4) x (instructions of a warp): one1 for a warp of single modes,
 // one2 of pairs.  Pairs issue fewer in all but come in coarser units, and reach
 // 95% of the pipe's rate (single modes 99%): 128^2 modes over 47 levels take 106
-// us as singles, 191 us as pairs, 384^2 modes 885 and 821.  One block per SM
+// us as singles, 191 us as pairs, 384^2 modes 885 and 821.  Up to some 9,000
+// modes (fewer than two warps an SM) four lanes share a mode where the kernel
+// has that form: lane4 instructions a lane.  One block per SM
 // holds all its warps, at most 16: the number per SM is exact (small blocks are
 // not dealt evenly), they share a level table, and more work goes in rounds of
 // equal size, as a last round of fewer than four warps runs at their own rate.
 // 512^2 modes over 207 levels: 3035 us in blocks of one warp, 2858 so (97% of
 // the pipe for 14 warps an SM); the accurate sweep of 512^2 over 104: 869, 805.
 struct Sweep64Launch {
-    bool pairs;
+    bool pairs, lanes;
     int threads;
     unsigned blocks;
 };
 
-static Sweep64Launch sweep64_launch(const SolveGeom &g, int nsm, double one1, double one2)
+static Sweep64Launch sweep64_launch(const SolveGeom &g, int nsm, double one1, double one2, double lane4 = 1e30)
 {
     auto per_sm = [&](int64_t n) { return ((n + 31) / 32 + nsm - 1) / nsm; };
     auto units = [&](int64_t n) { return (double)std::max<int64_t>(per_sm(n), 4); };
     const int64_t n2 = sweep_items(g.nlx, g.nly).n;
     Sweep64Launch l;
     l.pairs = units(n2) * one2 < 0.95 * units(g.nsolved) * one1;
-    const int64_t n = l.pairs ? n2 : g.nsolved, w = per_sm(n);
+    l.lanes = units(4 * g.nsolved) * lane4 < 0.95 * std::min(units(n2) * one2, units(g.nsolved) * one1);
+    const int64_t n = l.lanes ? 4 * g.nsolved : l.pairs ? n2 : g.nsolved, w = per_sm(n);
     const int64_t rounds = (w + SWEEP64_THREADS / 32 - 1) / (SWEEP64_THREADS / 32);
     l.threads = 32 * (int)((w + rounds - 1) / rounds);
     l.blocks = (unsigned)std::min<int64_t>((n + 31) / 32, nsm);
@@ -960,9 +1032,12 @@ cudaError_t launch_sweep64(const SolveGeom &g, const double *lvtab, const int *s
     if (first_on_device(attr)) {
         cudaFuncSetAttribute(sweep64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(sweep64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(sweep64_lanes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     }
-    const Sweep64Launch l = sweep64_launch(g, nsm, 68, 124);
-    if (l.pairs)
+    const Sweep64Launch l = sweep64_launch(g, nsm, 68, 124, 33);
+    if (l.lanes)
+        sweep64_lanes_kernel<<<l.blocks, l.threads, smem, st>>>(g, lvtab, slot, modes, q0spec, snap, top, err);
+    else if (l.pairs)
         sweep64_kernel<2><<<l.blocks, l.threads, smem, st>>>(g, lvtab, slot, modes, q0spec, snap, top, err);
     else
         sweep64_kernel<1><<<l.blocks, l.threads, smem, st>>>(g, lvtab, slot, modes, q0spec, snap, top, err);

@@ -106,6 +106,8 @@ def test_training_step_tiles(n, offset):
     (512, 560, True, 8),            # even, with the unpaired Nyquist row and column
     (460, 512, False, [0, 3, 8]),   # a source spectrum and several output levels
     (20, 6, False, [0, 3, 8]),      # one mode per thread, fewer modes than a block
+    (97, 101, True, 8),             # four lanes per mode, a last warp partly filled
+    (120, 140, False, [0, 3, 8]),   # ... two warps of them a scheduler
     (3, 2, True, 4),                # the smallest grids
 ])
 def test_fp64_sweep_items(nx, ny, footprint, levels):
