@@ -192,8 +192,9 @@ struct HostBuffers {
     size_t ws_bytes = 0;
     double *srf = nullptr;
     size_t srf_bytes = 0;
-    double *conc = nullptr, *flx = nullptr;
+    double *out = nullptr;  // conc, then flx
     size_t out_bytes = 0;
+    int *status = nullptr;  // pinned
     cudaStream_t stream = nullptr;
 };
 // A pinned upload buffer; its event marks the last copy out of it.
@@ -568,22 +569,23 @@ int solve_impl(const bldfm_desc *d, const double *srf_dev, const double *z, cons
     int *slot = (int *)(w + L.slot);
     const int nz = g.nz;
 
-    // stage per-call host data: level tables and the snapshot schedule
-    const size_t lv64b = (size_t)std::max(nz - 1, 0) * BLDFM_LV64 * 8;
-    const size_t lv32b = (size_t)std::max(nz - 1, 0) * BLDFM_LV32 * 4;
+    // stage per-call host data as the head of the workspace holds it (status
+    // word, level tables, snapshot schedule, k = 0 values): one upload
     const size_t slotb = (size_t)nz * 4;
     const size_t eigb = (shoot || g.analytic) ? (size_t)g.nsolved * 16 : 0;
     const size_t dcb = (size_t)g.nlvls * 32;
-    const size_t off_lv32 = al(lv64b), off_slot = off_lv32 + al(lv32b), off_dc = off_slot + al(slotb),
-                 off_eig = off_dc + al(dcb);
+    const size_t off_lv64 = L.lv64 - L.err, off_lv32 = L.lv32 - L.err, off_slot = L.slot - L.err,
+                 off_dc = L.dc - L.err, off_eig = L.eig - L.err;
     StageSlot *slt = nullptr;
     if ((rc = acquire_stage(dc, off_eig + al(eigb) + 256, &slt)) != BLDFM_OK) return rc;
     char *sg = (char *)slt->buf;
     timers_begin(dc);
+    memset(sg, 0, off_lv64);
+    double *slv = (double *)(sg + off_lv64);
     if (!f64 && g.footprint)
-        hx_level_dz_w(nz, z, prof, (double *)sg);  // the FP32 footprint reads only what the k = 0 values use
+        hx_level_dz_w(nz, z, prof, slv);  // the FP32 footprint reads only what the k = 0 values use
     else
-        hx_level_table(nz, z, prof, (double *)sg);
+        hx_level_table(nz, z, prof, slv);
     if (!f64) {
         if (g.iso)
             hx_level_table32_iso(nz, z, prof, g.ex, g.ey, (float *)(sg + off_lv32), nullptr);
@@ -613,16 +615,12 @@ int solve_impl(const bldfm_desc *d, const double *srf_dev, const double *z, cons
             hdc[2] = qr;
             hdc[3] = qi;
         } else {
-            hx_dc_values(nz, (const double *)sg, hp.slot.data(), q0r, 0.0, d->srf_bg_conc,
+            hx_dc_values(nz, slv, hp.slot.data(), q0r, 0.0, d->srf_bg_conc,
                          g.precision == BLDFM_PREC_SINGLE, g.nlvls, 0, hdc);
         }
     }
 
-    CK(cudaMemsetAsync(err, 0, 64, st));
-    if (lv64b) CK(cudaMemcpyAsync(lv64, sg, lv64b, cudaMemcpyHostToDevice, st));
-    if (!f64 && lv32b) CK(cudaMemcpyAsync(lv32, sg + off_lv32, lv32b, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(slot, sg + off_slot, slotb, cudaMemcpyHostToDevice, st));
-    if (g.footprint) CK(cudaMemcpyAsync(dcv, sg + off_dc, dcb, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(w + L.err, sg, g.footprint ? off_dc + dcb : off_slot + slotb, cudaMemcpyHostToDevice, st));
     // every spectrum entry is written unless some output slot stays empty
     // (duplicate levels) or the analytic branch runs
     const size_t specb = (size_t)g.nlvls * g.nlx * g.nly * (f64 ? 16 : 8);
@@ -1805,15 +1803,15 @@ int bldfm_solve_host(const bldfm_desc *d, const double *srf_flx_host, const doub
             CK(cudaMalloc(&hb.ws, (size_t)pi.workspace_bytes));
             hb.ws_bytes = (size_t)pi.workspace_bytes;
         }
+        if (!hb.status) CK(cudaHostAlloc(&hb.status, sizeof(int), cudaHostAllocDefault));
         const size_t outb = (size_t)nlvls * pi.out_ny * pi.out_nx * sizeof(double);
-        if (outb > hb.out_bytes) {
-            if (hb.conc) cudaFree(hb.conc);
-            if (hb.flx) cudaFree(hb.flx);
-            hb.conc = hb.flx = nullptr;
-            CK(cudaMalloc(&hb.conc, std::max<size_t>(outb, 8)));
-            CK(cudaMalloc(&hb.flx, std::max<size_t>(outb, 8)));
-            hb.out_bytes = outb;
+        if (2 * outb > hb.out_bytes || !hb.out) {
+            if (hb.out) cudaFree(hb.out);
+            hb.out = nullptr;
+            CK(cudaMalloc(&hb.out, std::max<size_t>(2 * outb, 16)));
+            hb.out_bytes = 2 * outb;
         }
+        double *flx_dev = hb.out + outb / sizeof(double);
         const double *srf_dev = nullptr;
         if (!d->footprint) {
             if (!srf_flx_host) return BLDFM_ERR_ARG;
@@ -1827,16 +1825,20 @@ int bldfm_solve_host(const bldfm_desc *d, const double *srf_flx_host, const doub
             CK(cudaMemcpyAsync(hb.srf, srf_flx_host, sb, cudaMemcpyHostToDevice, hb.stream));
             srf_dev = hb.srf;
         }
-        rc = solve_impl(d, srf_dev, z_host, prof_host, levels_host, nlvls, hb.conc, hb.flx, hb.ws, hb.ws_bytes,
+        rc = solve_impl(d, srf_dev, z_host, prof_host, levels_host, nlvls, hb.out, flx_dev, hb.ws, hb.ws_bytes,
                         hb.stream);
         if (rc != BLDFM_OK) return rc;
-        if (outb) {
-            CK(cudaMemcpyAsync(conc_host, hb.conc, outb, cudaMemcpyDeviceToHost, hb.stream));
-            CK(cudaMemcpyAsync(flx_host, hb.flx, outb, cudaMemcpyDeviceToHost, hb.stream));
+        // the status word goes to pinned memory: queued, while a copy to the
+        // caller's pageable arrays returns when it is done
+        CK(cudaMemcpyAsync(hb.status, hb.ws, sizeof(int), cudaMemcpyDeviceToHost, hb.stream));
+        if (outb && flx_host == conc_host + outb / sizeof(double)) {
+            CK(cudaMemcpyAsync(conc_host, hb.out, 2 * outb, cudaMemcpyDeviceToHost, hb.stream));
+        } else if (outb) {
+            CK(cudaMemcpyAsync(conc_host, hb.out, outb, cudaMemcpyDeviceToHost, hb.stream));
+            CK(cudaMemcpyAsync(flx_host, flx_dev, outb, cudaMemcpyDeviceToHost, hb.stream));
         }
-        int err = 0;
-        CK(cudaMemcpyAsync(&err, hb.ws, sizeof(int), cudaMemcpyDeviceToHost, hb.stream));
         CK(cudaStreamSynchronize(hb.stream));
+        const int err = *hb.status;
         if (err != 0) return err == BLDFM_ERR_NONFINITE ? BLDFM_ERR_NONFINITE : BLDFM_ERR_TIMEOUT;
         return BLDFM_OK;
     });
