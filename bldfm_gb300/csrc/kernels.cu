@@ -1048,7 +1048,10 @@ cudaError_t launch_combine64(const SolveGeom &g, const uint32_t *modes, const do
                              const double2 *top, double2 *Xp, double2 *Xq, cudaStream_t st)
 {
     if (g.nsolved == 0) return cudaSuccess;
-    const int threads = 256;
+    // small blocks: a thread's work is a serial chain per level, and few modes
+    // in large ones leave SMs idle (14,250 modes, nine levels: 23 us in blocks
+    // of 256, 17 so; 4,096 modes and one level: 11, 6)
+    const int threads = 64;
     const unsigned blocks = (unsigned)((g.nsolved + threads - 1) / threads);
     combine64_kernel<<<blocks, threads, 0, st>>>(g, modes, eig, snap, top, Xp, Xq);
     return LAUNCH_CHECK();
