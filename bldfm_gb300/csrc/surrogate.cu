@@ -193,8 +193,9 @@ struct Mlp {
     float *P = nullptr, *G = nullptr, *m = nullptr, *v = nullptr;
     MlpBlocks blk = {};
     MlpTrainBuf buf = {};
-    float *loss = nullptr;
+    float *loss = nullptr;  // and the status word behind it
     int *err = nullptr;
+    float *host_tail = nullptr;  // pinned: loss, status
     std::vector<void *> allocs;  // every device allocation, freed with the object
     Mlp() = default;
     Mlp(const Mlp &) = delete;
@@ -202,6 +203,7 @@ struct Mlp {
     ~Mlp()
     {
         for (void *p : allocs) cudaFree(p);
+        if (host_tail) cudaFreeHost(host_tail);
     }
 };
 
@@ -271,7 +273,8 @@ int bldfm_surrogate_create(int32_t batch, uint64_t seed, void **handle)
         const size_t B = (size_t)batch;
         bool ok = mlp_alloc(*M, &M->P, MLP_NPARAM) && mlp_alloc(*M, &M->G, MLP_NPARAM) &&
                   mlp_alloc(*M, &M->m, MLP_NPARAM) && mlp_alloc(*M, &M->v, MLP_NPARAM) &&
-                  mlp_alloc(*M, &M->loss, 1) && mlp_alloc(*M, &M->err, 1) &&
+                  mlp_alloc(*M, &M->loss, 2) &&
+                  cudaHostAlloc(&M->host_tail, 8, cudaHostAllocDefault) == cudaSuccess &&
                   mlp_alloc(*M, &M->buf.part_w, mlp_train_part_w(batch, M->nsm)) &&
                   mlp_alloc(*M, &M->buf.part_o, mlp_train_part_o(batch, M->nsm)) &&
                   mlp_alloc(*M, &M->buf.Xp, B * 32) && mlp_alloc(*M, &M->buf.D[3], B * MLP_H);
@@ -282,6 +285,7 @@ int bldfm_surrogate_create(int32_t batch, uint64_t seed, void **handle)
                  mlp_alloc(*M, &M->buf.H[j], B * MLP_H) && mlp_alloc(*M, &M->buf.D[j], B * MLP_H) &&
                  mlp_alloc(*M, &M->buf.G[j], B * MLP_H);
         if (!ok) return BLDFM_ERR_CUDA;
+        M->err = (int *)(M->loss + 1);
         // He-scaled normal weights (Box-Muller on a 64-bit LCG), zero biases
         std::vector<float> p(MLP_NPARAM, 0.f);
         uint64_t s = seed * 6364136223846793005ULL + 1442695040888963407ULL;
@@ -340,11 +344,15 @@ int bldfm_surrogate_grads(void *handle, float *host_grads, float *host_loss)
     Mlp *M = (Mlp *)handle;
     if (!M) return BLDFM_ERR_ARG;
     if (cudaDeviceSynchronize() != cudaSuccess) return BLDFM_ERR_CUDA;
+    // loss and status to pinned memory, queued; the copy to the caller's
+    // pageable array behind it returns when both are there
+    if (cudaMemcpyAsync(M->host_tail, M->loss, 8, cudaMemcpyDeviceToHost, 0) != cudaSuccess) return BLDFM_ERR_CUDA;
     if (host_grads && cudaMemcpy(host_grads, M->G, MLP_NPARAM * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
         return BLDFM_ERR_CUDA;
-    if (host_loss && cudaMemcpy(host_loss, M->loss, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return BLDFM_ERR_CUDA;
+    if (cudaStreamSynchronize(0) != cudaSuccess) return BLDFM_ERR_CUDA;
+    if (host_loss) *host_loss = M->host_tail[0];
     int e = 0;
-    if (cudaMemcpy(&e, M->err, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return BLDFM_ERR_CUDA;
+    memcpy(&e, M->host_tail + 1, sizeof(e));
     return e != 0 ? BLDFM_ERR_TIMEOUT : BLDFM_OK;
 }
 
