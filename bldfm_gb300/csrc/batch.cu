@@ -1138,6 +1138,12 @@ int batch_xform_occupancy(int col, size_t smem)
 
 void prepare_batch_attributes()
 {
+    // An SM changes its split of L1 and shared memory only when it is empty.  The
+    // checks run beside the transform passes; with their own preference (mostly
+    // L1) the column pass waited on every SM that held some of the check (16
+    // fields of 512^2: column pass 85 us, 73 so; the call 593 -> 580)
+    for (const void *k : {(const void *)fp32_check_kernel, (const void *)sur_guard_kernel})
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     prepare_rx_attributes();
     cudaFuncSetAttribute(riccati32_batch_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(riccati32_batch_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
