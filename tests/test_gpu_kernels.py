@@ -45,7 +45,7 @@ def test_generic_radix_lengths(nx, ny, halo, footprint):
 
 
 @pytest.mark.parametrize("count,n", [(1, 1), (1, 2), (3, 1023), (2, 1024), (5, 4095), (3, 4097), (2, 70001),
-                                     (700, 33), (1, 1300003)])
+                                     (700, 33), (3, 65536), (3, 65537), (1, 1300003)])
 @pytest.mark.parametrize("phase", [0, 1])
 def test_point_measurement_remainders(count, n, phase):
     """Every remainder and both 8-byte phases against math.fsum of the exact
