@@ -1236,19 +1236,26 @@ cudaError_t launch_output_fft(const SolveGeom &g, const FftPlan &plx, const FftP
     return LAUNCH_CHECK();
 }
 
+static const int FWD_MAX_CASES = 65535;  // the grid's y limit
+
 cudaError_t launch_forward_batch(const FwdCase *cases, int n, int rows, size_t row_smem, int cols, size_t col_smem,
                                  cudaStream_t st)
 {
     set_fft_smem_attr<float>();
-    fwd_rows_batch_kernel<<<dim3(rows, n), 256, row_smem, st>>>(cases);
-    fwd_cols_batch_kernel<<<dim3(cols, n), 256, col_smem, st>>>(cases);
+    for (int i = 0; i < n; i += FWD_MAX_CASES) {
+        const int m = n - i < FWD_MAX_CASES ? n - i : FWD_MAX_CASES;
+        fwd_rows_batch_kernel<<<dim3(rows, m), 256, row_smem, st>>>(cases + i);
+        fwd_cols_batch_kernel<<<dim3(cols, m), 256, col_smem, st>>>(cases + i);
+    }
     return LAUNCH_CHECK();
 }
 
 cudaError_t launch_dc_batch(const FwdCase *cases, int n, int max_nz, cudaStream_t st)
 {
     set_fft_smem_attr<float>();
-    dc_partial_batch_kernel<<<dim3(DC_PARTS, n), 256, 0, st>>>(cases);
+    for (int i = 0; i < n; i += FWD_MAX_CASES)
+        dc_partial_batch_kernel<<<dim3(DC_PARTS, n - i < FWD_MAX_CASES ? n - i : FWD_MAX_CASES), 256, 0, st>>>(cases +
+                                                                                                              i);
     const size_t smem = (size_t)(max_nz > 1 ? max_nz - 1 : 1) * sizeof(double2) + (size_t)max_nz * sizeof(int);
     trapezoid_batch_kernel<<<n, 256, smem, st>>>(cases);
     return LAUNCH_CHECK();

@@ -130,6 +130,22 @@ def test_fp64_sweep_items(nx, ny, footprint, levels):
     assert relerr(c, oc) <= 1e-11 and relerr(f, of) <= 1e-11
 
 
+def test_batch_of_more_sources_than_a_grid_row():
+    """The forward passes take cases by the grid's y, which ends at 65,535: the
+    cases on both sides of it give what a batch of three gives (the same FP32
+    operations per case: a few ulp)."""
+    from bldfm_gb300.batch import solve_batch
+
+    three = [dict(ragged_kw(4, 2, 0, False), precision="single") for _ in range(3)]
+    for k, kw in enumerate(three):
+        kw["srf_flx"] = kw["srf_flx"] + k
+    ref = solve_batch(three)
+    res = solve_batch([three[k % 3] for k in range(65537)])
+    for k in (0, 1, 65533, 65534, 65535, 65536):
+        for a, b in zip(res[k][1:], ref[k % 3][1:]):
+            assert relerr(a, b) <= 16 * 2.0**-24
+
+
 @pytest.mark.parametrize("sizes", [
     [(4, 2)],                              # one line per block, fewer lines than blocks
     [(64, 48), (4, 2), (150, 302)],        # several cases: the grid is the largest case's
