@@ -25,6 +25,7 @@ ERR_TIMEOUT = -9
 ERR_NONFINITE = -10
 ERR_PROFILE = -11
 ERR_HOST = -12
+ERR_BUSY = -13
 
 PREC_SINGLE = 0
 PREC_DOUBLE = 1

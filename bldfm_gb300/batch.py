@@ -209,16 +209,18 @@ class BatchSolver:
         if t is None or tuple(t.shape) != a.shape:
             t = torch.empty(a.shape, dtype=torch.float64, device=self.device)
             self._srf[k] = t
-        # one core fills the library's staging ring at 28 GB/s (384 KB: 24 us
+        # one core fills a pinned buffer of the library at 28 GB/s (384 KB: 24 us
         # against 50 through a pinned tensor); from about 1 MB on torch's
-        # parallel copy into one is the faster
+        # parallel copy into one is the faster, and it takes what the library's
+        # buffers, filled with copies behind a busy stream, do not
         if a.nbytes <= 1 << 20:
             with torch.cuda.device(self.device):
-                _lib.check(_lib.load().bldfm_upload_async(t.data_ptr(), a.ctypes.data, a.nbytes,
-                                                          self.stream.cuda_stream), "solve_batch")
-        else:
-            with torch.cuda.stream(self.stream):
-                t.copy_(torch.from_numpy(a).pin_memory(), non_blocking=True)
+                st = _lib.load().bldfm_upload_async(t.data_ptr(), a.ctypes.data, a.nbytes, self.stream.cuda_stream)
+            if st != _lib.ERR_BUSY:
+                _lib.check(st, "solve_batch")
+                return t
+        with torch.cuda.stream(self.stream):
+            t.copy_(torch.from_numpy(a).pin_memory(), non_blocking=True)
         return t
 
     def prepare(self, cases, views=True):

@@ -203,7 +203,16 @@ struct StageSlot {
     size_t bytes = 0;
     cudaEvent_t ev = nullptr;
 };
-enum { NSTAGE = 8, NTIMER = 8, NTSETS = 1024 };
+// A pinned buffer of bldfm_upload_async, apart from the ring: what waits behind a
+// busy stream here holds up neither other streams' solves nor the library's lock.
+// `taken` from the choice of the slot until its copies are enqueued.
+struct UploadSlot {
+    void *buf = nullptr;
+    cudaEvent_t ev = nullptr;
+    std::atomic<bool> taken{false};
+};
+enum { NSTAGE = 8, NTIMER = 8, NTSETS = 1024, NUPLOAD = 8 };
+const size_t UPLOAD_BYTES = (size_t)1 << 20;
 // CUDA events of one solve's stage boundaries
 struct TimerSet {
     cudaEvent_t ev[NTIMER + 1] = {};
@@ -224,6 +233,7 @@ struct DeviceCache {
     std::map<std::vector<int>, int4 *> xband;
     StageSlot stage[NSTAGE];  // ring of pinned staging buffers
     int stage_next = 0;
+    UploadSlot upload[NUPLOAD];
     HostBuffers hb;
     // CUDA graphs of batches, keyed by the launch topology; each instance owns
     // the pinned buffer its upload node reads
@@ -252,6 +262,9 @@ DeviceCache &cache_for_current(int *status)
         if (dc.nsm <= 0) dc.nsm = 1;
         for (int i = 0; i < NSTAGE; ++i)
             if (cudaEventCreateWithFlags(&dc.stage[i].ev, cudaEventDisableTiming) != cudaSuccess)
+                *status = BLDFM_ERR_CUDA;
+        for (int i = 0; i < NUPLOAD; ++i)
+            if (cudaEventCreateWithFlags(&dc.upload[i].ev, cudaEventDisableTiming) != cudaSuccess)
                 *status = BLDFM_ERR_CUDA;
         prepare_kernel_attributes();
         prepare_batch_attributes();
@@ -359,6 +372,22 @@ int acquire_stage(DeviceCache &dc, size_t bytes, StageSlot **out)
         sl.bytes = want;
     }
     *out = &sl;
+    return BLDFM_OK;
+}
+
+// Host data through a taken upload slot, without the library's lock; data of
+// more than one buffer waits for its own earlier part.
+int upload_through(UploadSlot &up, char *dst, const char *src, size_t bytes, cudaStream_t st)
+{
+    if (!up.buf && cudaHostAlloc(&up.buf, UPLOAD_BYTES, cudaHostAllocDefault) != cudaSuccess) return BLDFM_ERR_CUDA;
+    for (size_t o = 0; o < bytes; o += UPLOAD_BYTES) {
+        const size_t nb = std::min(UPLOAD_BYTES, bytes - o);
+        if (o > 0 && cudaEventSynchronize(up.ev) != cudaSuccess) return BLDFM_ERR_CUDA;
+        memcpy(up.buf, src + o, nb);
+        if (cudaMemcpyAsync(dst + o, up.buf, nb, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+            cudaEventRecord(up.ev, st) != cudaSuccess)
+            return BLDFM_ERR_CUDA;
+    }
     return BLDFM_OK;
 }
 
@@ -1625,6 +1654,7 @@ const char *bldfm_status_str(int s)
     case BLDFM_ERR_NONFINITE: return "non-finite values in the output";
     case BLDFM_ERR_PROFILE:
         return "z must be strictly increasing and the profiles finite with Kz > 0 and Kx, Ky >= 0";
+    case BLDFM_ERR_BUSY: return "every upload buffer holds a copy that is still in flight";
     case BLDFM_ERR_HOST: return "host-side failure (memory allocation or thread start)";
     default: return "unknown status";
     }
@@ -1657,23 +1687,23 @@ int bldfm_upload_async(void *dst, const void *src, size_t bytes, void *stream)
     return bldfm_guarded([&]() -> int {
         if (bytes == 0) return BLDFM_OK;
         if (!dst || !src) return BLDFM_ERR_ARG;
-        std::lock_guard<std::mutex> lk(g_mutex);
-        int status = BLDFM_OK;
-        DeviceCache &dc = cache_for_current(&status);
-        if (status != BLDFM_OK) return status;
-        // 1 MB at a time through the ring of staging buffers: the copy into one
-        // overlaps the transfer of the one before, and the ring stays small
-        const size_t chunk = (size_t)1 << 20;
-        for (size_t o = 0; o < bytes; o += chunk) {
-            const size_t nb = std::min(chunk, bytes - o);
-            StageSlot *slt = nullptr;
-            int rc = acquire_stage(dc, nb, &slt);
-            if (rc != BLDFM_OK) return rc;
-            memcpy(slt->buf, (const char *)src + o, nb);
-            CK(cudaMemcpyAsync((char *)dst + o, slt->buf, nb, cudaMemcpyHostToDevice, (cudaStream_t)stream));
-            CK(cudaEventRecord(slt->ev, (cudaStream_t)stream));
+        UploadSlot *up = nullptr;
+        {
+            std::lock_guard<std::mutex> lk(g_mutex);
+            int status = BLDFM_OK;
+            DeviceCache &dc = cache_for_current(&status);
+            if (status != BLDFM_OK) return status;
+            for (int i = 0; i < NUPLOAD && !up; ++i)
+                if (!dc.upload[i].taken.load(std::memory_order_acquire) &&
+                    cudaEventQuery(dc.upload[i].ev) == cudaSuccess)
+                    up = &dc.upload[i];
+            (void)cudaGetLastError();  // a copy in flight is no error
+            if (!up) return BLDFM_ERR_BUSY;
+            up->taken.store(true, std::memory_order_relaxed);
         }
-        return BLDFM_OK;
+        const int rc = upload_through(*up, (char *)dst, (const char *)src, bytes, (cudaStream_t)stream);
+        up->taken.store(false, std::memory_order_release);
+        return rc;
     });
 }
 

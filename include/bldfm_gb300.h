@@ -46,6 +46,7 @@ extern "C" {
                                         Kz <= 0 or Kx, Ky < 0 (checked on the host before any work) */
 #define BLDFM_ERR_HOST -12           /* host-side failure: memory allocation or thread start (a C++
                                         exception inside the library, caught at the entry point) */
+#define BLDFM_ERR_BUSY -13           /* bldfm_upload_async: no upload buffer is free, nothing was enqueued */
 
 /* ---- descriptor -------------------------------------------------------- */
 #define BLDFM_PREC_SINGLE 0 /* reference precision="single": spectra stored as complex64 */
@@ -171,10 +172,12 @@ int bldfm_stage_times(float *ms, int n);
  * buffer with it). */
 int bldfm_memcpy_async(void *dst, const void *src, size_t bytes, void *stream);
 
-/* Copy host data of any kind to the device on the caller's stream through the
- * library's pinned staging ring: src may be changed or freed as soon as the
- * call returns.  No reference counterpart (the sources of a batch go up with
- * it). */
+/* Copy host data of any kind to the device on the caller's stream through one
+ * of the library's pinned upload buffers (eight of 1 MB per device): src may be
+ * changed or freed as soon as the call returns.  It waits for no other stream:
+ * BLDFM_ERR_BUSY, with nothing enqueued, when every buffer still holds a copy
+ * in flight.  Data of more than 1 MB waits for its own first part.  No
+ * reference counterpart (the sources of a batch go up with it). */
 int bldfm_upload_async(void *dst, const void *src, size_t bytes, void *stream);
 
 /* Algorithmic flops of the FP32 Riccati sweep for one solved mode (an FMA

@@ -147,3 +147,56 @@ def test_solve_stream_matches_solve_batch():
             np.testing.assert_array_equal(rc, gc)
             np.testing.assert_array_equal(rf, gf)
             assert rc.dtype == gc.dtype
+
+
+def test_sources_behind_a_busy_stream_hold_up_nobody():
+    """A batch of more sources than the library has upload buffers, enqueued
+    behind work still running on its stream: the call returns at once, and so
+    does a solve on another stream; the results are those of an idle stream."""
+    import torch
+
+    from bldfm_gb300.batch import BatchSolver
+
+    base = _cases(3)[1]
+    cases = [dict(base, srf_flx=base["srf_flx"] * (1 + k)) for k in range(20)]
+    solver, other = BatchSolver(check=False), BatchSolver(check=False)
+
+    def outs(res):
+        return [t.clone() for pair in res for t in pair]
+
+    with torch.cuda.stream(solver.stream):
+        want = outs(solver.solve(cases))
+    other.solve(cases[:1])
+    torch.cuda.synchronize()
+    running = torch.cuda.Event()
+    with torch.cuda.stream(solver.stream):
+        torch.cuda._sleep(1_000_000_000)  # about half a second
+        running.record()
+        got = solver.solve(cases)
+        for _ in range(10):
+            other.solve(cases[:1])
+        other.stream.synchronize()
+        assert not running.query()
+        got = outs(got)
+    torch.cuda.synchronize()
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 1 << 17, (1 << 17) + 1, 500_000])
+def test_upload_copies_the_source_before_it_returns(n):
+    """bldfm_upload_async on both sides of its buffers' 1 MB, the source
+    overwritten as soon as the call returns."""
+    import torch
+
+    from bldfm_gb300 import _lib
+
+    src = np.random.default_rng(n).random(n)
+    want = src.copy()
+    dst = torch.zeros(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    _lib.check(_lib.load().bldfm_upload_async(dst.data_ptr(), src.ctypes.data, src.nbytes, s.cuda_stream))
+    src[:] = -1.0
+    s.synchronize()
+    np.testing.assert_array_equal(dst.cpu().numpy(), want)
