@@ -270,15 +270,19 @@ class BatchSolver:
                 self.stream.synchronize()
             self._out_buf = torch.empty(total, dtype=torch.float64, device=self.device)
 
-    def _fill(self, cases, metas, views, off=0, k0=0):
+    def _fill(self, cases, metas, views, off=0, k0=0, upload=True):
         """The C descriptors of cases whose outputs start at element off of the
-        output buffer; k0: place of the first one in its batch."""
+        output buffer; k0: place of the first one in its batch; upload=False:
+        for planning only, which reads no source."""
         n = len(cases)
         arr = (_lib.Case * n)()
         outs, keep = [], []
         base = self._out_buf.data_ptr()
         for k, ((d, shape, sz, footprint), zp, nz, levels, lv, lvp, zptr) in enumerate(metas):
-            srf = 0 if footprint else self._srf_dev(k0 + k, cases[k]["srf_flx"]).data_ptr()
+            if footprint:
+                srf = 0
+            else:
+                srf = self._srf_dev(k0 + k, cases[k]["srf_flx"]).data_ptr() if upload else base
             _CASE.pack_into(arr, k * _CASE.size, d, srf, zptr, zptr + 8 * nz, lvp, lv.size, 0, base + 8 * off,
                             base + 8 * (off + sz))
             if views:
@@ -320,12 +324,7 @@ class BatchSolver:
         if ws is not None and (len(prepared) <= 3 or ws.numel() >= prepared[3]):
             st = run()
         if st == _lib.ERR_WORKSPACE:
-            if len(prepared) > 3:
-                need = prepared[3]
-            else:
-                nb = ctypes.c_int64(0)
-                _lib.check(lib.bldfm_batch_plan(arr, n, self.opts, ctypes.byref(nb)), "solve_batch")
-                need = int(nb.value)
+            need = prepared[3] if len(prepared) > 3 else self._plan(arr)
             if ws is None or ws.numel() < need:
                 if ws is not None:  # an earlier batch on the stream may still use it
                     self.stream.synchronize()
@@ -334,17 +333,20 @@ class BatchSolver:
         _lib.check(st, "solve_batch")
         return ws
 
+    def _plan(self, arr):
+        """Workspace bytes of a batch; raises what the library refuses it for."""
+        nb = ctypes.c_int64(0)
+        _lib.check(_lib.load().bldfm_batch_plan(arr, len(arr), self.opts, ctypes.byref(nb)), "solve_batch")
+        return int(nb.value)
+
     def _workspaces(self):
         """(workspace, cases) of each part of the last batch."""
         return list(zip([self._ws] + self._more_ws, self._parts))
 
     def prepare_cached(self, cases):
         """:meth:`prepare` plus the workspace size, for repeated solves."""
-        lib = _lib.load()
         arr, outs, keep = self.prepare(cases)
-        need = ctypes.c_int64(0)
-        _lib.check(lib.bldfm_batch_plan(arr, len(cases), self.opts, ctypes.byref(need)), "solve_batch")
-        return (arr, outs, keep, int(need.value))
+        return (arr, outs, keep, self._plan(arr))
 
     def status(self):
         """Device status word of the last batch (0, or a BLDFM_ERR_* code),
@@ -441,8 +443,16 @@ def _enqueue_parts(solver, cases):
     if nparts < 2:
         return _enqueue_batch(solver, cases)
     n = len(cases)
-    solver._reserve(sum(sizes))
-    nout = 8 * sum(sizes)
+    # a refused case leaves the solver, the last batch's outputs among it, as it
+    # was: every case is described and planned before the first part runs (which
+    # the library itself plans before it enqueues anything)
+    metas = solver._metas(cases)
+    offs = [0]
+    for m in metas:
+        offs.append(offs[-1] + 2 * m[0][2])
+    solver._reserve(offs[-1])
+    solver._plan(solver._fill(cases[cuts[1] :], metas[cuts[1] :], False, upload=False)[0])
+    nout = 8 * offs[-1]
     nhead = 64 + 16 * n  # as one batch's; then 64 bytes with the status word of each further part
     block = torch.empty(nout + nhead + 64 * (nparts - 1), dtype=torch.uint8, pin_memory=True)
     base, dev = block.data_ptr(), solver._out_buf.data_ptr()
@@ -450,35 +460,30 @@ def _enqueue_parts(solver, cases):
         solver._copy_stream = torch.cuda.Stream(device=solver.device)
     cs = solver._copy_stream
     solver._more_ws += [None] * (nparts - 1 - len(solver._more_ws))
-    shapes, keep, off = [], [], 0
+    shapes, keep, parts = [], [], []
     try:
         for i in range(nparts):
             lo, hi = cuts[i], cuts[i + 1]
-            part = cases[lo:hi]
-            metas = solver._metas(part)
-            prepared = solver._fill(part, metas, False, off, lo)
+            prepared = solver._fill(cases[lo:hi], metas[lo:hi], False, offs[lo], lo)
             if i == 0:
                 ws = solver._ws = solver._run(prepared, solver._ws)
             else:
                 ws = solver._more_ws[i - 1] = solver._run(prepared, solver._more_ws[i - 1])
-            cs.wait_stream(solver.stream)
-            cnt = 2 * sum(m[0][2] for m in metas)
-            _memcpy(base + 8 * off, dev + 8 * off, 8 * cnt, cs)
-            _memcpy(base + (nout if i == 0 else nout + nhead + 64 * (i - 1)), ws.data_ptr(), 64, cs)
-            _memcpy(base + nout + 64 + 16 * lo, ws.data_ptr() + 64, 16 * (hi - lo), cs)
-            off += cnt
+            parts.append(hi - lo)
             shapes += prepared[1]
             keep += prepared[2]
+            cs.wait_stream(solver.stream)
+            _memcpy(base + 8 * offs[lo], dev + 8 * offs[lo], 8 * (offs[hi] - offs[lo]), cs)
+            _memcpy(base + (nout if i == 0 else nout + nhead + 64 * (i - 1)), ws.data_ptr(), 64, cs)
+            _memcpy(base + nout + 64 + 16 * lo, ws.data_ptr() + 64, 16 * (hi - lo), cs)
+    except BaseException:
+        cs.synchronize()  # the copies into the pinned block, which goes now
+        raise
     finally:
-        # the solver's stream goes on only after the copies, and so does a
-        # caller that gets an exception: the pinned block is theirs until then
-        solver.stream.wait_stream(cs)
-        if len(keep) < n:
-            solver.stream.synchronize()
-    solver.out_elems = off
-    solver._parts = [b - a for a, b in zip(cuts, cuts[1:])]
-    solver._keep = keep
-    return (solver, cases, shapes, keep, block[: 8 * off].view(torch.float64), block[nout:])
+        solver.stream.wait_stream(cs)  # it goes on only after the copies
+        if parts:  # what runs, or ran, is the solver's last batch
+            solver._parts, solver._keep, solver.out_elems = parts, keep, offs[sum(parts)]
+    return (solver, cases, shapes, keep, block[:nout].view(torch.float64), block[nout:])
 
 
 def _finish_batch(pending):

@@ -214,3 +214,85 @@ def test_serving_tiles(count, size):
     for i in range(0, count, 13):
         c, f = sur.solve_prepared(sur.prepare(**items[i]))
         assert relerr(outs[i][0], c.cpu().numpy()) < 1e-6 and relerr(outs[i][1], f.cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("bad", ["modes", "profile"])
+def test_refused_parts_leave_the_last_batch(monkeypatch, bad):
+    """A large batch whose last case is refused, by its description or by its
+    profiles, is refused before anything runs: outputs on the device, status word
+    and error statements stay the last batch's."""
+    from bldfm_gb300 import batch as B
+
+    z, p = O.vertical_profiles(8, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    cases = [dict(srf_flx=np.full((48, 64), 0.5 + i), z=z, profiles=p, domain=(256.0, 192.0), levels=8, modes=(64, 48),
+                  meas_pt=(3.0, 2.0 + i), footprint=i % 2 == 0, halo=8.0, precision="double") for i in range(6)]
+    s = B.BatchSolver()
+    outs = [t for pair in s.solve(cases) for t in pair]
+    want, est = [t.cpu() for t in outs], s.error_estimates(6)
+    monkeypatch.setattr(B, "PART_BYTES", 1 << 16)
+    assert len(B._split_batch([B._output_bound(kw) for kw in cases])) > 2
+    neg = tuple(-a for a in p)
+    last = dict(cases[0], modes=(5, 4)) if bad == "modes" else dict(cases[0], profiles=neg)
+    with pytest.raises(ValueError):
+        B.solve_batch(cases[:0:-1] + [last], solver=s)
+    s.stream.synchronize()
+    for a, b in zip(want, outs):
+        np.testing.assert_array_equal(a, b.cpu())
+    assert s.status() == 0
+    np.testing.assert_array_equal(s.error_estimates(6), est)
+
+
+def test_failure_between_parts_keeps_what_ran(monkeypatch):
+    """A part that fails after the first has run: the solver's last batch is the
+    parts that ran, and the next batch is as good as ever."""
+    from bldfm_gb300 import batch as B
+
+    z, p = O.vertical_profiles(8, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    cases = [dict(srf_flx=np.zeros((48, 64)), z=z, profiles=p, domain=(256.0, 192.0), levels=8, modes=(64, 48),
+                  meas_pt=(3.0, 2.0 + i), footprint=True, halo=8.0, precision="double") for i in range(6)]
+    s = B.BatchSolver()
+    whole = B.solve_batch(cases, solver=s)
+    monkeypatch.setattr(B, "PART_BYTES", 1 << 16)
+    cuts = B._split_batch([B._output_bound(kw) for kw in cases])
+    run, calls = s._run, []
+
+    def failing(prepared, ws):
+        calls.append(len(prepared[0]))
+        if len(calls) == 2:
+            raise RuntimeError("second part")
+        return run(prepared, ws)
+
+    monkeypatch.setattr(s, "_run", failing)
+    with pytest.raises(RuntimeError, match="second part"):
+        B.solve_batch(cases, solver=s)
+    monkeypatch.undo()
+    assert s._parts == [cuts[1]] and s.status() == 0
+    np.testing.assert_allclose(s.error_estimates(cuts[1]), whole.error_estimates[: cuts[1]], rtol=32 * 2.0**-23)
+    for (_, c0, f0), (_, c1, f1) in zip(whole, B.solve_batch(cases, solver=s)):
+        np.testing.assert_array_equal(c0, c1)
+        np.testing.assert_array_equal(f0, f1)
+
+
+@pytest.mark.parametrize("at", [2, 5])
+def test_status_of_every_part(monkeypatch, at):
+    """A non-finite source in a middle or the last part: the call reports it, the
+    solver's status word too, and the next batch is clean."""
+    from bldfm_gb300 import _lib
+    from bldfm_gb300 import batch as B
+
+    z, p = O.vertical_profiles(8, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    cases = [dict(srf_flx=np.full((48, 64), 0.5), z=z, profiles=p, domain=(256.0, 192.0), levels=8, modes=(64, 48),
+                  meas_pt=(3.0, 2.0), footprint=False, halo=8.0, precision="double") for _ in range(6)]
+    monkeypatch.setattr(B, "PART_BYTES", 1 << 16)
+    cuts = B._split_batch([B._output_bound(kw) for kw in cases])
+    assert len(cuts) == 5 and cuts[1] <= 2 and cuts[-2] <= 5
+    bad = [dict(kw) for kw in cases]
+    bad[at]["srf_flx"] = bad[at]["srf_flx"].copy()
+    bad[at]["srf_flx"][3, 5] = np.nan
+    s = B.BatchSolver()
+    for _ in range(2):
+        with pytest.raises(FloatingPointError):
+            B.solve_batch(bad, solver=s)
+        assert s.status() == _lib.ERR_NONFINITE
+        B.solve_batch(cases, solver=s)
+        assert s.status() == 0
