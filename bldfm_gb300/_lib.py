@@ -173,6 +173,7 @@ _SIGS = {
         ctypes.c_int,
         [ctypes.POINTER(Case), ctypes.c_int32, ctypes.POINTER(BatchOpts), ctypes.POINTER(ctypes.c_int64)],
     ),
+    "bldfm_batch_check": (ctypes.c_int, [ctypes.POINTER(Case), ctypes.c_int32]),
     "bldfm_solve_batch": (
         ctypes.c_int,
         [ctypes.POINTER(Case), ctypes.c_int32, ctypes.POINTER(BatchOpts), _P, ctypes.c_size_t, _P],

@@ -273,7 +273,7 @@ class BatchSolver:
     def _fill(self, cases, metas, views, off=0, k0=0, upload=True):
         """The C descriptors of cases whose outputs start at element off of the
         output buffer; k0: place of the first one in its batch; upload=False:
-        for planning only, which reads no source."""
+        for a check only, which reads no source."""
         n = len(cases)
         arr = (_lib.Case * n)()
         outs, keep = [], []
@@ -324,7 +324,12 @@ class BatchSolver:
         if ws is not None and (len(prepared) <= 3 or ws.numel() >= prepared[3]):
             st = run()
         if st == _lib.ERR_WORKSPACE:
-            need = prepared[3] if len(prepared) > 3 else self._plan(arr)
+            if len(prepared) > 3:
+                need = prepared[3]
+            else:
+                nb = ctypes.c_int64(0)
+                _lib.check(lib.bldfm_batch_plan(arr, n, self.opts, ctypes.byref(nb)), "solve_batch")
+                need = int(nb.value)
             if ws is None or ws.numel() < need:
                 if ws is not None:  # an earlier batch on the stream may still use it
                     self.stream.synchronize()
@@ -333,20 +338,17 @@ class BatchSolver:
         _lib.check(st, "solve_batch")
         return ws
 
-    def _plan(self, arr):
-        """Workspace bytes of a batch; raises what the library refuses it for."""
-        nb = ctypes.c_int64(0)
-        _lib.check(_lib.load().bldfm_batch_plan(arr, len(arr), self.opts, ctypes.byref(nb)), "solve_batch")
-        return int(nb.value)
-
     def _workspaces(self):
         """(workspace, cases) of each part of the last batch."""
         return list(zip([self._ws] + self._more_ws, self._parts))
 
     def prepare_cached(self, cases):
         """:meth:`prepare` plus the workspace size, for repeated solves."""
+        lib = _lib.load()
         arr, outs, keep = self.prepare(cases)
-        return (arr, outs, keep, self._plan(arr))
+        need = ctypes.c_int64(0)
+        _lib.check(lib.bldfm_batch_plan(arr, len(cases), self.opts, ctypes.byref(need)), "solve_batch")
+        return (arr, outs, keep, int(need.value))
 
     def status(self):
         """Device status word of the last batch (0, or a BLDFM_ERR_* code),
@@ -411,7 +413,7 @@ def _output_bound(kw):
     never larger than the source grid."""
     lv = kw.get("levels", 0)
     ny, nx = np.shape(kw["srf_flx"])[-2:]
-    return 2 * int(ny) * int(nx) * max(1, int(np.size(lv)))
+    return 2 * int(ny) * int(nx) * (1 if type(lv) is int else max(1, int(np.size(lv))))
 
 
 def _split_batch(sizes):
@@ -433,7 +435,8 @@ def _enqueue_parts(solver, cases):
     its own, and each part's outputs go back on a second stream while the next
     part is prepared and computed.  Sixteen towers of 256^2 to 1024^2 (98 MB of
     results): as one batch 530 us of copying followed the last kernel, as four
-    parts 140 (2121 -> 1927 us)."""
+    parts 140 (2121 -> 1927 us).  Every case is described and checked before the
+    first part runs, which costs 30 us of it."""
     try:
         sizes = [_output_bound(kw) for kw in cases]
         cuts = _split_batch(sizes)
@@ -444,18 +447,18 @@ def _enqueue_parts(solver, cases):
         return _enqueue_batch(solver, cases)
     n = len(cases)
     # a refused case leaves the solver, the last batch's outputs among it, as it
-    # was: every case is described and planned before the first part runs (which
-    # the library itself plans before it enqueues anything)
+    # was: every case is described and checked before the first part runs (whose
+    # own cases the library checks before it enqueues anything)
     metas = solver._metas(cases)
     offs = [0]
     for m in metas:
         offs.append(offs[-1] + 2 * m[0][2])
     solver._reserve(offs[-1])
-    solver._plan(solver._fill(cases[cuts[1] :], metas[cuts[1] :], False, upload=False)[0])
+    rest = solver._fill(cases[cuts[1] :], metas[cuts[1] :], False, upload=False)[0]
+    _lib.check(_lib.load().bldfm_batch_check(rest, len(rest)), "solve_batch")
     nout = 8 * offs[-1]
     nhead = 64 + 16 * n  # as one batch's; then 64 bytes with the status word of each further part
-    block = torch.empty(nout + nhead + 64 * (nparts - 1), dtype=torch.uint8, pin_memory=True)
-    base, dev = block.data_ptr(), solver._out_buf.data_ptr()
+    dev = solver._out_buf.data_ptr()
     if solver._copy_stream is None:
         solver._copy_stream = torch.cuda.Stream(device=solver.device)
     cs = solver._copy_stream
@@ -472,6 +475,9 @@ def _enqueue_parts(solver, cases):
             parts.append(hi - lo)
             shapes += prepared[1]
             keep += prepared[2]
+            if i == 0:
+                block = torch.empty(nout + nhead + 64 * (nparts - 1), dtype=torch.uint8, pin_memory=True)
+                base = block.data_ptr()
             cs.wait_stream(solver.stream)
             _memcpy(base + 8 * offs[lo], dev + 8 * offs[lo], 8 * (offs[hi] - offs[lo]), cs)
             _memcpy(base + (nout if i == 0 else nout + nhead + 64 * (i - 1)), ws.data_ptr(), 64, cs)

@@ -759,6 +759,15 @@ struct BatchBuild {
     std::vector<int> cpck, rpck;             // lines per column / row CTA of each case
 };
 
+int batch_case_check(const bldfm_case &c)
+{
+    if (c.desc.mode != BLDFM_MODE_FP32 || c.desc.analytic) return BLDFM_ERR_UNSUPPORTED;
+    if (!c.z_host || !c.prof_host || !c.levels_host || !c.conc_dev || !c.flx_dev ||
+        (!c.desc.footprint && !c.srf_flx_dev))
+        return BLDFM_ERR_ARG;
+    return BLDFM_OK;
+}
+
 int batch_build(const bldfm_case *cs, int n, const bldfm_batch_opts *opts, DeviceCache *dc, BatchBuild &B,
                 size_t extra_blob = 0)
 {
@@ -783,12 +792,8 @@ int batch_build(const bldfm_case *cs, int n, const bldfm_batch_opts *opts, Devic
     std::vector<int> status(n, BLDFM_OK);
     HostPool::get().run(n, [&](int k) {
         const bldfm_case &c = cs[k];
-        if (c.desc.mode != BLDFM_MODE_FP32 || c.desc.analytic)
-            status[k] = BLDFM_ERR_UNSUPPORTED;
-        else if (!c.z_host || !c.prof_host || !c.levels_host || !c.conc_dev || !c.flx_dev ||
-                 (!c.desc.footprint && !c.srf_flx_dev))
-            status[k] = BLDFM_ERR_ARG;
-        else
+        status[k] = batch_case_check(c);
+        if (status[k] == BLDFM_OK)
             status[k] = make_plan(&c.desc, c.z_host, c.prof_host, c.levels_host, c.nlvls, B.hp[k]);
     });
     for (int k = 0; k < n; ++k)
@@ -1885,6 +1890,21 @@ int bldfm_batch_plan(const bldfm_case *cases, int32_t ncases, const bldfm_batch_
         *workspace_bytes = (int64_t)B.total;
         return BLDFM_OK;
     });
+}
+
+int bldfm_batch_check(const bldfm_case *cases, int32_t ncases)
+{
+    if (!cases || ncases < 1) return BLDFM_ERR_ARG;
+    for (int k = 0; k < ncases; ++k) {
+        const bldfm_case &c = cases[k];
+        const int rc = batch_case_check(c), nz = c.desc.nz;
+        if (rc != BLDFM_OK) return rc;
+        if (nz < 1 || c.nlvls < 1) return BLDFM_ERR_ARG;
+        for (int l = 0; l < c.nlvls; ++l)
+            if (c.levels_host[l] < -(int64_t)nz || c.levels_host[l] >= nz) return BLDFM_ERR_ARG;
+        if (hx_check_profiles(nz, c.z_host, c.prof_host) != 0) return BLDFM_ERR_PROFILE;
+    }
+    return BLDFM_OK;
 }
 
 int bldfm_solve_batch(const bldfm_case *cases, int32_t ncases, const bldfm_batch_opts *opts, void *workspace,

@@ -231,6 +231,12 @@ typedef struct bldfm_batch_opts {
 int bldfm_batch_plan(const bldfm_case *cases, int32_t ncases,
                      const bldfm_batch_opts *opts, int64_t *workspace_bytes);
 
+/* Status of the first case whose pointers, levels or profiles a batch would be
+ * refused for, its descriptor having passed bldfm_plan, without planning the
+ * batch: some 1 us a case.  For a caller that enqueues a large batch in parts
+ * and must know of a refusal before the first one runs. */
+int bldfm_batch_check(const bldfm_case *cases, int32_t ncases);
+
 /* Enqueue a batch on stream; returns once enqueued.  The int32 at workspace
  * offset 0 holds the device status after completion.  A workspace smaller
  * than the batch needs gives BLDFM_ERR_WORKSPACE before anything is

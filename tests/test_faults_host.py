@@ -229,3 +229,36 @@ def test_batch_plan_from_many_threads():
         t.join()
     assert not errs
     assert len(got) == 400 and all(r == want[i] for i, r in got)
+
+
+def test_batch_check_finds_what_planning_refuses_a_case_for():
+    """The check of a batch's cases by themselves: pointers, levels and profiles,
+    in any place, with the status that planning gives."""
+    lib = _lib.load()
+    z, prof = _good()
+    out = np.zeros(1)
+    good = np.array([len(z) - 1], dtype=np.int64)
+    opts = _lib.BatchOpts(0, 0, 0, 0, 0)
+
+    def both(k, zz=z, p=prof, lv=good, mode="fp32", conc=True):
+        arr = (_lib.Case * 3)()
+        for i, c in enumerate(arr):
+            bad = i == k
+            c.desc = make_desc((48, 64), len(z), (128.0, 96.0), (64, 48), (40.0, 50.0), 0.0, True, False, None,
+                               "double", mode if bad else "fp32")
+            c.z_host, c.prof_host = (zz if bad else z).ctypes.data, (p if bad else prof).ctypes.data
+            c.levels_host, c.nlvls = (lv if bad else good).ctypes.data, 1
+            c.conc_dev = out.ctypes.data if conc or not bad else None
+            c.flx_dev = out.ctypes.data
+        nb = ctypes.c_int64(0)
+        return lib.bldfm_batch_check(arr, 3), lib.bldfm_batch_plan(arr, 3, ctypes.byref(opts), ctypes.byref(nb))
+
+    assert both(-1) == (0, 0)
+    for k in range(3):
+        for _, zz, p in _bad_profiles():
+            assert both(k, zz=zz, p=p) == (_lib.ERR_PROFILE, _lib.ERR_PROFILE)
+        for bad in (len(z), -len(z) - 1):
+            assert both(k, lv=np.array([bad], dtype=np.int64)) == (_lib.ERR_ARG, _lib.ERR_ARG)
+        assert both(k, mode="fp64") == (_lib.ERR_UNSUPPORTED, _lib.ERR_UNSUPPORTED)
+        assert both(k, conc=False) == (_lib.ERR_ARG, _lib.ERR_ARG)
+    assert lib.bldfm_batch_check(None, 1) == _lib.ERR_ARG
