@@ -190,8 +190,8 @@ def steady_state_transport_solver(
     d = make_desc(shape, nz, domain, modes, meas_pt, srf_bg_conc, footprint, analytic, halo, precision, mode)
     info = _lib.PlanInfo()
     _lib.check(lib.bldfm_plan(d, int(lv.size), info), "steady_state_transport_solver")
-    # back to back, as on the device: one copy
-    conc, flx = np.empty((2, lv.size, info.out_ny, info.out_nx), dtype=np.float64)
+    conc = np.empty((lv.size, info.out_ny, info.out_nx), dtype=np.float64)
+    flx = np.empty_like(conc)
     src = None if footprint else np.ascontiguousarray(srf_flx, dtype=np.float64)
     st = lib.bldfm_solve_host(
         d, _lib.ptr(src), _lib.ptr(zz), _lib.ptr(prof), _lib.ptr(lv), int(lv.size), _lib.ptr(conc), _lib.ptr(flx)

@@ -296,3 +296,19 @@ def test_status_of_every_part(monkeypatch, at):
         assert s.status() == _lib.ERR_NONFINITE
         B.solve_batch(cases, solver=s)
         assert s.status() == 0
+
+
+@pytest.mark.parametrize("mode", ["fp64", "fp64r"])
+@pytest.mark.parametrize("nx,ny,levels", [(64, 48, 8), (7, 5, [2, 8]), (512, 400, [0, 8])])
+def test_single_solve_outputs_own_their_memory(mode, nx, ny, levels):
+    """A caller that keeps one output of a single solve keeps no memory of the
+    other: each array's memory is its own and no larger."""
+    from bldfm_gb300 import steady_state_transport_solver
+
+    z, p = O.vertical_profiles(8, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    _, c, f = steady_state_transport_solver(np.zeros((ny, nx)), z, p, (4.0 * nx, 4.0 * ny), levels,
+                                            modes=(nx & ~1, ny & ~1), footprint=True, halo=8.0, precision="double",
+                                            mode=mode)
+    owners = [a if a.base is None else a.base for a in (c, f)]
+    assert owners[0] is not owners[1]
+    assert all(o.base is None and o.nbytes == a.nbytes for o, a in zip(owners, (c, f)))
