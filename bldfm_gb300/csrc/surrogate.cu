@@ -223,9 +223,9 @@ cudaError_t gemm(const uint16_t *A, const uint16_t *Bop, int tiles, int K, int s
                  cudaStream_t st)
 {
     const size_t smem = tc_gemm_smem(256);
-    static uint64_t attr = 0;
-    if (first_on_device(attr))
-        cudaFuncSetAttribute(tc_gemm_kernel<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static std::atomic<uint64_t> attr{0};
+    const cudaError_t c = set_dynamic_smem(attr, tc_gemm_kernel<Epi>, smem);
+    if (c != cudaSuccess) return c;
     tc_gemm_kernel<Epi><<<dim3(tiles, splits), 128, smem, st>>>(A, Bop, K, 256, epi, err);
     return cudaGetLastError();
 }

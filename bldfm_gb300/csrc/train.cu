@@ -881,12 +881,10 @@ cudaError_t launch_mlp_train(const float *X, const float *T, const float *w, int
     a.inv_n = 1.0f / n;
     a.err = err;
     const int grid = step_grid(a.pairs, nsm);
-    static uint64_t step_attr = 0;
-    cudaError_t e = cudaSuccess;
-    if (first_on_device(step_attr) &&
-        (e = cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STEP_SMEM)) !=
-            cudaSuccess)
-        return e;
+    static std::atomic<uint64_t> step_attr{0}, grad_attr{0};
+    cudaError_t e = set_dynamic_smem(step_attr, mlp_step_kernel, STEP_SMEM);
+    if (e == cudaSuccess) e = set_dynamic_smem(grad_attr, mlp_grad_kernel, GRAD_SMEM);
+    if (e != cudaSuccess) return e;
     mlp_step_kernel<<<grid, STEP_THREADS, STEP_SMEM, st>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     GradArgs ga;
@@ -902,11 +900,6 @@ cudaError_t launch_mlp_train(const float *X, const float *T, const float *w, int
         off += (size_t)ga.splits[j] * (j > 0 ? PB_H : PB_0);
     }
     ga.err = err;
-    static uint64_t attr = 0;
-    if (first_on_device(attr) &&
-        (e = cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAD_SMEM)) !=
-            cudaSuccess)
-        return e;
     mlp_grad_kernel<<<cta, GRAD_THREADS, GRAD_SMEM, st>>>(ga);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     UpdateArgs ua;
