@@ -207,6 +207,7 @@ _SIGS = {
         ctypes.c_int,
         [ctypes.c_int32, _P, _P, _P, ctypes.POINTER(ctypes.c_size_t), _P, _P, _P, ctypes.c_size_t, _P],
     ),
+    "bldfm_selftest_train_status": (ctypes.c_int, [_P, ctypes.c_int32]),
     "bldfm_selftest_wait_timeout": (ctypes.c_int, [ctypes.c_int64, ctypes.POINTER(ctypes.c_int32),
                                                     ctypes.POINTER(ctypes.c_int64)]),
     "bldfm_surrogate_plan": (ctypes.c_int, [ctypes.POINTER(Desc), ctypes.c_int32, ctypes.POINTER(ctypes.c_int64)]),

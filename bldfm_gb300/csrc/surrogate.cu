@@ -338,6 +338,18 @@ int bldfm_surrogate_params(void *handle, float *host_out, const float *host_in)
     return BLDFM_OK;
 }
 
+// status word of the network's device waits, for checks of the failure path
+int bldfm_selftest_train_status(void *handle, int32_t status)
+{
+    Mlp *M = (Mlp *)handle;
+    if (!M) return BLDFM_ERR_ARG;
+    if (cudaDeviceSynchronize() != cudaSuccess ||
+        cudaMemcpy(M->err, &status, sizeof(status), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaDeviceSynchronize() != cudaSuccess)
+        return BLDFM_ERR_CUDA;
+    return BLDFM_OK;
+}
+
 // gradients of the last training step and its loss
 int bldfm_surrogate_grads(void *handle, float *host_grads, float *host_loss)
 {

@@ -765,15 +765,17 @@ struct UpdateArgs {
     int splits[4];
     size_t off[4];
     int no;  // partials of the output layer
+    const int *err;
     MlpAdam m;
     MlpBlocks blk;
 };
 
-// one thread per parameter (and one for the loss)
+// one thread per parameter (and one for the loss).  After a wait that ran out,
+// in this step or before it, the partial sums are incomplete: nothing changes.
 __global__ void __launch_bounds__(256) mlp_update_kernel(const UpdateArgs a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > MLP_NPARAM) return;
+    if (i > MLP_NPARAM || *a.err != 0) return;
     const float *p;
     int cnt, stride;
     if (i >= MLP_OFF_W4) {
@@ -910,6 +912,7 @@ cudaError_t launch_mlp_train(const float *X, const float *T, const float *w, int
         ua.off[j] = ga.off[j];
     }
     ua.no = grid;
+    ua.err = err;
     ua.m = adam;
     ua.blk = blk;
     mlp_update_kernel<<<(MLP_NPARAM + 256) / 256, 256, 0, st>>>(ua);

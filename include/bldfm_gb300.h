@@ -304,6 +304,12 @@ int bldfm_point_measurement(const double *f_dev, const double *g_dev,
  * time the bounded wait took in *wait_ns_host. */
 int bldfm_selftest_wait_timeout(int64_t limit, int32_t *status_host, int64_t *wait_ns_host);
 
+/* The same for training: sets the status word of a network's device waits (0,
+ * or BLDFM_ERR_TIMEOUT as a wait that ran out does).  While it is not 0 a
+ * training step changes neither gradients, moments nor parameters, and
+ * bldfm_surrogate_grads reports it. */
+int bldfm_selftest_train_status(void *handle, int32_t status);
+
 /* Training data of the surrogate (no reference counterpart): a pool of
  * nondimensional MOST met cases (s1 = z_m / L, s2 = ln(z_m / z0)) on the
  * n-level stretched grid of vertical_profiles (src/bldfm/pbl_model.py:8-204,

@@ -56,3 +56,31 @@ def test_training_reduces_loss():
     net.train_step(Xd, Td, wd, 0.0)
     _, l1 = net.grads()
     assert l1 < 0.05 * l0, (l0, l1)
+
+
+def test_step_after_a_timeout_changes_nothing():
+    """A wait that ran out leaves partial sums behind: the step's update, and those
+    of later steps, leave parameters and moments alone, and grads reports it."""
+    import torch
+
+    from bldfm_gb300 import _lib
+    from bldfm_gb300.mlp import MLP
+
+    rng = np.random.default_rng(7)
+    X, T, w = (torch.from_numpy(rng.uniform(-1, 1, (256, k)).astype(np.float32)).cuda() for k in (8, 4, 4))
+    net, twin = MLP(batch=256, seed=3), MLP(batch=256, seed=3)
+    status = _lib.load().bldfm_selftest_train_status
+    for m in (net, twin):
+        m.train_step(X, T, w, 1e-3)
+    p = net.params()
+    assert status(net.h, _lib.ERR_TIMEOUT) == 0
+    net.train_step(X, T, w, 1e-3)
+    with pytest.raises(RuntimeError, match="timed out"):
+        net.grads()
+    np.testing.assert_array_equal(net.params(), p)
+    # cleared, the gradients are those of a network that never failed: the
+    # operand blocks were left alone too
+    assert status(net.h, 0) == 0
+    for m in (net, twin):
+        m.train_step(X, T, w, 0.0)
+    np.testing.assert_array_equal(net.grads()[0], twin.grads()[0])
