@@ -2,23 +2,24 @@
 // src/bldfm/utils.py:80-92, np.sum(f * g)) for a batch of (footprint, flux)
 // pairs: out[b] = sum_i f[b][i] g[b][i] in FP64.
 //
-// The field is HBM-bound (16 bytes read per point, nothing written) as long as
-// the FP64 pipe keeps up: at 2 lanes per clock and SM it passes about 0.53 T
-// instructions/s, while HBM delivers 0.42 T points/s, so a point may cost no
-// more than 1.25 FP64 instructions.  A compensated sum per point took five
-// (195 us for 64 x 512^2 points, 1.37 TB/s).  Here a thread adds 16 points in
-// two chains of 8 FMAs (products unrounded) and only the sum of those 16 goes
-// through the compensated accumulator: 1.31 instructions a point.  The short
-// chains' roundings are independent and average out over the blocks.  Each batch
-// entry is split over the CTAs of one grid row, each with a contiguous range;
-// the CTA combines its threads in a fixed order, and the cluster or a second
-// kernel (one warp per entry) adds the per-CTA partials in a fixed order, so the
-// result is deterministic (no atomics).  The last few additions, which hold
-// nearly all of the error, keep their rounding errors: relative error over 64
-// fields of 512^2 5.3e-17, 400 of 300^2 5.9e-17 (the rounding of the result
-// itself; 5.4e-17 and 8.3e-17 with Kahan's sum per point and plain trees), for
-// 2 us of the 59 that a call on 64 x 512^2 takes.  numpy's pairwise sum differs
-// at the level of its own rounding (about log2(n) eps).
+// HBM (16 bytes read per point, nothing written) and the FP64 pipe bound it about
+// evenly: at 2 lanes per clock and SM the pipe passes some 0.53 T instructions/s
+// and HBM delivers 0.42 T points/s, 1.25 instructions a point.  A compensated
+// sum per point took five (195 us for 64 x 512^2 points, 1.37 TB/s).  Here a
+// thread adds 16 points in two chains of 8 FMAs (products unrounded) and only the
+// sum of those 16 goes through the compensated accumulator: 1.31 instructions a
+// point, 59 us.  Each batch entry is split over the CTAs of one grid row, each
+// with a contiguous range; the CTA combines its threads in a fixed order, and the
+// cluster or a second kernel (one warp per entry) adds the per-CTA partials in a
+// fixed order, so the result is deterministic (no atomics).
+//
+// Every addition over threads, warps and CTAs keeps its rounding error.  Worst
+// case in u = 2^-53 of sum |f g|, at any n: 12 (chain 8, join of the two chains 1,
+// compensated sum 2, result 1); a compensated sum per point with a plain tree
+// over the threads has 13.  Footprints against flux maps: 64 fields of 512^2
+// 5.3e-17, 400 of 300^2 5.2e-17, the rounding of the result itself (5.4e-17 and
+// 8.3e-17 with that tree).  numpy's pairwise sum differs at the level of its own
+// rounding (about log2(n) eps).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -40,10 +41,10 @@ struct Kahan {
     }
 };
 
-// The sums of the last levels carry their rounding errors along (TwoSum: exact):
-// an error made in one of M equal partial sums weighs 1 / sqrt(M) in the result,
-// so the few last additions hold nearly all of it.  The chain from one addition
-// to the next is one instruction, Kahan's is four.
+// A sum that carries its rounding errors along (TwoSum: exact).  An error made in
+// one of M equal partial sums weighs 1 / sqrt(M) in the result, so the last
+// additions would hold nearly all of it.  The chain from one addition to the
+// next is one instruction, Kahan's is four.
 struct TwoSum {
     double s = 0.0, e = 0.0;
     __device__ __forceinline__ void add(double x)
@@ -53,16 +54,29 @@ struct TwoSum {
         e = __dadd_rn(e, __dadd_rn(__dsub_rn(s, __dsub_rn(t, b)), __dsub_rn(x, b)));
         s = t;
     }
+    // lanes l and l + off, for off, off / 2 ... 1, in lane 0
+    __device__ __forceinline__ void add_lanes(int off)
+    {
+        for (; off > 0; off >>= 1) {
+            const double s2 = __shfl_down_sync(0xffffffffu, s, off), e2 = __shfl_down_sync(0xffffffffu, e, off);
+            add(s2);
+            e = __dadd_rn(e, e2);
+        }
+    }
     __device__ __forceinline__ double sum() const { return __dadd_rn(s, e); }
 };
 
-const int MEAS_UNROLL = 8;  // 16-byte loads of each field in flight per thread
-const int MEAS_CTAS = 4;    // resident CTAs per SM the grid is sized for (at most 64 registers a thread)
+const int MEAS_UNROLL = 8;  // pairs of points per compensated addition
+const int MEAS_CTAS = 4;    // resident CTAs per SM the grid is sized for; their 64 registers a thread hold some of
+                            // a block's 16 loads of 16 bytes in flight, not all
 // Fields of up to 65,536 points take at most eight CTAs, one cluster, which adds
 // its partial sums itself: one launch instead of two (31 -> 26 us a call).  With
 // more points a CTA than this it takes longer than the second launch (a single
 // field of 131,044 points: 46 us with its synchronisation, 43 over the device).
-// Batches that leave an entry no more than eight CTAs at any size take it too.
+// Batches that leave an entry no more than eight CTAs at any size take it too: 100
+// fields of 512^2 132 us (320 with a second launch and a compensated sum per
+// point), 305, which get one CTA each, 323 (998), 607 421 (1572), 100 of 1024^2
+// 363 (1137).
 const int MEAS_CLUSTER = 8, MEAS_CTA_POINTS = 8192;
 
 // not .aligned: thread 0 comes from a branch of its own
@@ -119,18 +133,17 @@ __global__ void __launch_bounds__(MEAS_THREADS, MEAS_CTAS)
         for (int64_t i = (int64_t)blockIdx.x * MEAS_THREADS + threadIdx.x; i < n; i += step)
             k.add(__dmul_rn(__ldg(fb + i), __ldg(gb + i)));
     }
-    // a warp's threads in a tree, the warps' sums with their errors
-    double v = __dadd_rn(k.s, -k.c);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, off));
-    __shared__ double ss[MEAS_THREADS / 32];
-    if ((threadIdx.x & 31) == 0) ss[threadIdx.x >> 5] = v;
+    // the threads' sums with their errors: eight per lane of one warp, then its lanes
+    __shared__ double ss[MEAS_THREADS];
+    ss[threadIdx.x] = __dadd_rn(k.s, -k.c);
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         TwoSum t;
+        t.s = ss[threadIdx.x];
 #pragma unroll
-        for (int w = 0; w < MEAS_THREADS / 32; ++w) t.add(ss[w]);
-        ss[0] = t.sum();
+        for (int w = 1; w < MEAS_THREADS / 32; ++w) t.add(ss[threadIdx.x + 32 * w]);
+        t.add_lanes(16);
+        if (threadIdx.x == 0) ss[0] = t.sum();
     }
     if (CLUSTER) {
         cluster_sync();
@@ -175,12 +188,7 @@ __global__ void __launch_bounds__(128) meas_final_kernel(const double *__restric
     if (b >= nbatch) return;
     TwoSum k;
     for (int i = lane; i < nparts; i += 32) k.add(part[(size_t)b * nparts + i]);
-    // as many levels as lanes hold partials
-    for (int off = nparts > 16 ? 16 : nparts > 8 ? 8 : 4; off > 0; off >>= 1) {
-        const double s2 = __shfl_down_sync(0xffffffffu, k.s, off), e2 = __shfl_down_sync(0xffffffffu, k.e, off);
-        k.add(s2);
-        k.e = __dadd_rn(k.e, e2);
-    }
+    k.add_lanes(nparts > 16 ? 16 : nparts > 8 ? 8 : 4);  // as many levels as lanes hold partials
     if (lane == 0) out[b] = k.sum();
 }
 

@@ -312,3 +312,39 @@ def test_single_solve_outputs_own_their_memory(mode, nx, ny, levels):
     owners = [a if a.base is None else a.base for a in (c, f)]
     assert owners[0] is not owners[1]
     assert all(o.base is None and o.nbytes == a.nbytes for o, a in zip(owners, (c, f)))
+
+
+@pytest.mark.parametrize("n", [65536, 4_000_000])  # one cluster; partial sums of the whole device
+@pytest.mark.parametrize("phase", [0, 1])
+@pytest.mark.parametrize("values", ["absorbed", "cancelling"])
+def test_point_measurement_worst_case(n, phase, values):
+    """Products that a plain addition loses, where a thread's chain of eight FMAs,
+    the join of its two chains and the sums over threads each meet them, and
+    sums that cancel within a thread's 16 points.  Bound in u = 2^-53 of the sum
+    of magnitudes: 8 for the chain, 1 for the join, 2 for the compensated sum, 1
+    for the result (13 for a compensated sum per point and a plain tree over 256
+    threads: product 1, sum 2, tree 8, partials 2)."""
+    import torch
+
+    from bldfm_gb300.utils import point_measurement_batch
+
+    lead = phase  # a field at an odd 8-byte phase has one leading point, then pairs
+    a = np.zeros(n)
+    pairs = a[lead:lead + 2 * ((n - lead) // 2)].reshape(-1, 2)
+    if values == "absorbed":
+        d = 0.99 * 2.0**-53
+        pairs[0] = 1.0, d                   # thread 0's chains; the second is lost in their join
+        pairs[256:2048:256, 0] = d          # ... and the first chain's seven further FMAs
+        pairs[[16, 8, 4, 2, 1], 0] = d      # the lanes a tree over the warp adds to lane 0
+        pairs[32:256:32, 0] = d             # ... and over the warps
+    else:
+        rng = np.random.default_rng(n)
+        m = len(pairs) // 512  # a thread's consecutive pairs are 256 apart
+        big = 10.0 ** rng.uniform(6, 9, (m, 1, 256, 1))
+        pairs[: 512 * m].reshape(m, 2, 256, 2)[:] = big * np.array([1.0, -1.0]).reshape(1, 2, 1, 1)
+        pairs += rng.uniform(-1, 1, pairs.shape)
+    f = torch.ones(n + 1, dtype=torch.float64, device="cuda")[phase:phase + n].view(1, n)
+    g = torch.empty(n + 1, dtype=torch.float64, device="cuda")[phase:phase + n].view(1, n)
+    g.copy_(torch.from_numpy(a).view(1, n))
+    out = float(point_measurement_batch(f, g)[0])
+    assert abs(out - math.fsum(a)) <= 12 * 2.0**-53 * math.fsum(np.abs(a))
