@@ -537,7 +537,8 @@ cudaError_t launch_sur_guard(const BatchCase *cases, int n, const int64_t *prefi
 // from |k| z_m < 4, 1.2% of the modes), so those modes take the exact FP32
 // sweep and the network serves the rest.  CTA b of case k (block0 <= b <
 // block0 + its CTAs) stages the level table in shared memory and sweeps box
-// positions j = 512 (b - block0) + t and j + 256 of the half box, two modes
+// positions j = SUR_LOWBAND_MODES (b - block0) + t and j + SUR_LOWBAND_THREADS
+// of the half box, two modes
 // in the lanes of packed f32x2 operations (ricc_rc_pair, which rounds as the
 // guard's ricc_rc_value does):
 //   j < by            kx = 0, ky = j + 1,

@@ -97,7 +97,8 @@ cudaError_t launch_sur_guard(const BatchCase *cases, int n, const int64_t *prefi
 // reaches an even mode count's Nyquist frequency, the unpaired modes of the
 // Nyquist column kx = -nlx/2 and row ky = -nly/2; two per thread, 128 per
 // CTA; modes outside the disc are skipped.  CTAs of two warps fit beside the
-// network's on an SM (alone, eight warps a CTA would be 4% faster).
+// network's on an SM; a single footprint, whose band runs alone, takes them as
+// well (512^2: 126 us, 129 with eight warps a CTA).
 #define SUR_LOWBAND_THREADS 64
 #define SUR_LOWBAND_MODES (2 * SUR_LOWBAND_THREADS)  // box positions per CTA
 struct __align__(16) LowBandCase {

@@ -63,18 +63,10 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-__device__ __forceinline__ float gelu_d(float z)
-{
-    const float z2 = z * z;
-    const float t = tanh_approx(GELU_C * fmaf(GELU_A * z2, z, z));
-    return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * GELU_C * fmaf(3.0f * GELU_A, z2, 1.0f);
-}
-
 // device views of a trained MLP for the fused serving kernel: FP32
-// parameters and the BF16 core-matrix blocks of Wt_1..3 (256 x 256 each)
+// parameters and the BF16 core-matrix blocks of Wt_1..3 / 2 (256 x 256 each)
 struct MlpServing {
     const float *P;
-    const uint16_t *Wt[3];  // 256 x 256 core-matrix blocks
-    const uint16_t *Wq[3];  // half of the same as four contiguous 128 x 128 quarters (N half, K half)
+    const uint16_t *Wq[3];  // four contiguous 128 x 128 quarters (N half, K half)
 };
 int mlp_serving_view(void *handle, MlpServing *out);

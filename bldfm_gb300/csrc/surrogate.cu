@@ -219,14 +219,13 @@ bool mlp_alloc(Mlp &M, T **p, size_t count)
 void mlp_free(Mlp *M) { delete M; }
 
 template <class Epi>
-cudaError_t gemm(const uint16_t *A, const uint16_t *Bop, int tiles, int K, int splits, Epi epi, int *err,
-                 cudaStream_t st)
+cudaError_t gemm(const uint16_t *A, const uint16_t *Bop, int tiles, int K, Epi epi, int *err, cudaStream_t st)
 {
     const size_t smem = tc_gemm_smem(256);
     static std::atomic<uint64_t> attr{0};
     const cudaError_t c = set_dynamic_smem(attr, tc_gemm_kernel<Epi>, smem);
     if (c != cudaSuccess) return c;
-    tc_gemm_kernel<Epi><<<dim3(tiles, splits), 128, smem, st>>>(A, Bop, K, 256, epi, err);
+    tc_gemm_kernel<Epi><<<tiles, 128, smem, st>>>(A, Bop, K, 256, epi, err);
     return cudaGetLastError();
 }
 
@@ -243,7 +242,7 @@ cudaError_t mlp_forward(Mlp &M, const float *X, int n, float *Y, cudaStream_t st
         e.W4 = M.P + MLP_OFF_W4;
         e.b4 = M.P + MLP_OFF_B4;
         e.Y = j == 3 ? Y : nullptr;
-        cudaError_t c = gemm(M.buf.H[j - 1], M.blk.Wt[j - 1], tiles, MLP_H, 1, e, M.err, st);
+        cudaError_t c = gemm(M.buf.H[j - 1], M.blk.Wt[j - 1], tiles, MLP_H, e, M.err, st);
         if (c != cudaSuccess) return c;
     }
     return cudaGetLastError();
@@ -416,7 +415,6 @@ int mlp_serving_view(void *handle, MlpServing *out)
     if (!M || !out) return BLDFM_ERR_ARG;
     out->P = M->P;
     for (int j = 0; j < 3; ++j) {
-        out->Wt[j] = M->blk.Wt[j];
         out->Wq[j] = M->blk.Wq[j];
     }
     return BLDFM_OK;

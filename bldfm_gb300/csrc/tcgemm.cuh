@@ -11,8 +11,7 @@
 #define TC_BLOCK_ROWS 128
 #define TC_N 256
 
-// Grid: blockIdx.x = 128-row tile of A, blockIdx.y = split of the K chunks
-// (split-K: CTA y handles chunks [y * cps, (y + 1) * cps)).  The epilogue gets
+// Grid: one CTA per 128-row tile of A.  The epilogue gets
 // epi.row(row, col0, v[32], tile_smem) for every 32-column slice, then, after
 // a barrier, epi.finish(tile, tile_smem) cooperatively; tile_smem is the
 // A-operand staging area (128 x KC bf16), free once the MMAs are done.
@@ -40,21 +39,18 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const uint16_t *__restr
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     const int nchunks = K / KC;
-    const int cps = (nchunks + gridDim.y - 1) / gridDim.y;
-    const int c0 = blockIdx.y * cps, c1 = min(nchunks, c0 + cps);
     const int tile = blockIdx.x;
     const uint32_t abytes = (uint32_t)TC_BLOCK_ROWS * KC * 2, bbytes = (uint32_t)TC_N * KC * 2;
     const uint32_t idesc = tc_idesc_bf16(TC_BLOCK_ROWS, TC_N);
     const uint32_t sbo = (uint32_t)(KC / 8) * 128;
     int issued = 0;  // MMA commits issued (for the drain on failure)
-    for (int c = c0; c < c1; ++c) {
-        const int it = c - c0;
+    for (int c = 0; c < nchunks; ++c) {
         if (threadIdx.x == 0) {
             tc_expect_tx(&bar_load, abytes + bbytes);
             tc_bulk_load(sA, Ablk + ((size_t)tile * nchunks + c) * TC_BLOCK_ROWS * KC, abytes, &bar_load);
             tc_bulk_load(sB, Bblk + (size_t)c * TC_N * KC, bbytes, &bar_load);
         }
-        if (!tc_mbar_wait(&bar_load, (uint32_t)(it & 1))) fail = 1;
+        if (!tc_mbar_wait(&bar_load, (uint32_t)(c & 1))) fail = 1;
         __syncthreads();
         if (fail) break;
         if (threadIdx.x == 0) {
@@ -62,11 +58,11 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const uint16_t *__restr
             const uint32_t a0 = tc_smem(sA), b0 = tc_smem(sB);
             for (int s = 0; s < KC / 16; ++s)
                 tc_mma(tmem, tc_desc(a0 + s * 256, 128, sbo), tc_desc(b0 + s * 256, 128, sbo), idesc,
-                       (it > 0 || s > 0) ? 1u : 0u);
+                       (c > 0 || s > 0) ? 1u : 0u);
             tc_commit(&bar_mma);
         }
-        issued = it + 1;
-        if (!tc_mbar_wait(&bar_mma, (uint32_t)(it & 1))) fail = 1;
+        issued = c + 1;
+        if (!tc_mbar_wait(&bar_mma, (uint32_t)(c & 1))) fail = 1;
         __syncthreads();
         if (fail) break;
     }

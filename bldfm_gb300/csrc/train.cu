@@ -18,8 +18,9 @@
 // 0.67 GB through L2 and HBM (activations, dZ, gelu', each written and read
 // once; 100 us at the HBM rate); and in the step kernel the CUDA cores: 16
 // packed FP32 operations and four tanh per two activations, 3.4 us for every
-// layer of every tile pair (55 us in all).  Measured: step 147 us, gradients
-// 54 us, update 16 us.  The layer-by-layer form before it (one launch per
+// layer of every tile pair (55 us in all).  Measured: step 144 us, gradients
+// 53 us, update 16 us; the step kernel's 96 registers a thread (18 warps) spill
+// some 40 words.  The layer-by-layer form before it (one launch per
 // GEMM, transposed copies of every operand, FP32 activations through HBM,
 // shuffled column sums, an atomic per gradient element) took 1,280 us.
 #include "devattr.h"
@@ -52,10 +53,10 @@ __device__ __forceinline__ uint4 pack8(const float *v)
                       pack_bf16x2(v[6], v[7]));
 }
 
-// h = gelu(z) and g = gelu'(z) for two values, each with the rounding of its
-// scalar form (gelu_f, gelu_d as compiled): the bf16 roundings downstream turn
-// one changed last bit in 10^4 into a changed activation, which moves a small
-// batch's gradient by 5e-5
+// h = gelu(z) and g = gelu'(z) for two values.  h rounds as gelu_f does; g takes
+// its tanh's argument as c (z + (a z^2) z), rounded after each of these, and h's
+// as z (c + (c a) z^2): the bf16 roundings downstream turn one changed last bit
+// in 10^4 into a changed activation, which moves a small batch's gradient by 5e-5
 __device__ __forceinline__ void gelu_both(float2 z, float2 &h, float2 &g)
 {
     auto c2 = [](float v) { return make_float2(v, v); };
