@@ -98,6 +98,8 @@ def _batch_inputs(cases):
         for kw in cases:
             z, p = kw["z"], kw["profiles"]
             nz = len(z)
+            if len(p) != 5:  # an iterator, which can be read once, has no length
+                break
             u, v, kx, ky, kz = p
             if not len(u) == len(v) == len(kx) == len(ky) == len(kz) == nz:
                 break

@@ -148,3 +148,20 @@ def test_prepare_fills_the_case_array():
         off += 2 * sz
     assert s.out_elems == off
     assert arr[0].desc.xmax == 80.0 and arr[1].desc.xmax == 90.0
+
+
+def test_batch_inputs_take_iterators_of_profiles_once():
+    """Profiles given as an iterator, beside a case that is not packed with the
+    others (scalar profiles): each is read once and packed as it is alone."""
+    from bldfm_gb300 import batch as B
+
+    p = _case()["profiles"]
+    scalar = _case(profiles=(1.0, 2.0, 3.0, 3.0, 3.0))
+    want = [B._host_inputs(_case())[0], B._host_inputs(scalar)[0]]
+    for cases in ([_case(profiles=iter(p)), scalar], [scalar, _case(profiles=map(np.asarray, p))]):
+        got = B._batch_inputs(cases)
+        order = want if cases[1] is scalar else want[::-1]
+        for g, w in zip(got, order):
+            np.testing.assert_array_equal(g[0], w)
+    one = B._batch_inputs([_case(profiles=(a for a in p))])
+    np.testing.assert_array_equal(one[0][0], want[0])
