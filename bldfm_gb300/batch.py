@@ -448,6 +448,7 @@ def _enqueue_parts(solver, cases):
     if nparts < 2:
         return _enqueue_batch(solver, cases)
     n = len(cases)
+    cases = [cases[k] for k in range(n)]  # any sequence
     # a refused case leaves the solver, the last batch's outputs among it, as it
     # was: every case is described and checked before the first part runs (whose
     # own cases the library checks before it enqueues anything)

@@ -348,3 +348,20 @@ def test_point_measurement_worst_case(n, phase, values):
     g.copy_(torch.from_numpy(a).view(1, n))
     out = float(point_measurement_batch(f, g)[0])
     assert abs(out - math.fsum(a)) <= 12 * 2.0**-53 * math.fsum(np.abs(a))
+
+
+def test_parts_of_any_sequence(monkeypatch):
+    """A large batch in a sequence that has no slices goes in parts as a list does."""
+    from collections import deque
+
+    from bldfm_gb300 import batch as B
+
+    z, p = O.vertical_profiles(8, 6.0, (2.0, -1.5), ustar=0.3, mol=-40.0)
+    cases = [dict(srf_flx=np.zeros((48, 64)), z=z, profiles=p, domain=(256.0, 192.0), levels=8, modes=(64, 48),
+                  meas_pt=(3.0, 2.0 + i), footprint=True, halo=8.0, precision="double") for i in range(6)]
+    whole = B.solve_batch(cases)
+    monkeypatch.setattr(B, "PART_BYTES", 1 << 16)
+    assert len(B._split_batch([B._output_bound(kw) for kw in cases])) > 2
+    for (_, c0, f0), (_, c1, f1) in zip(whole, B.solve_batch(deque(cases))):
+        np.testing.assert_array_equal(c0, c1)
+        np.testing.assert_array_equal(f0, f1)
